@@ -68,7 +68,7 @@ class Scratch:
         z = lambda *s, dt=torch.float32: torch.zeros(*s, dtype=dt, device=device)
         return Scratch(accum=z(accum_rows, accum_cols), tickets=z(8192, dt=torch.int32),
                        part_o=z(attn_slots), part_ml=z(attn_slots // 32), attn_tickets=z(8192, dt=torch.int32),
-                       status=z(4, dt=torch.int32), partials=z(148 * 2 * 128 * 32))
+                       status=z(4, dt=torch.int32), partials=z(148 * 2 * 128 * 128))
 
 
     def reset(self) -> None:
@@ -188,7 +188,9 @@ def gemm(pw: PackedWeight, x: torch.Tensor, out: torch.Tensor, *, epi: int = EPI
          tp: torch.Tensor | None = None) -> None:
     """Tensor-core path: out[M, N] (+)= x[M, K] @ dequant(W)^T, any M."""
     accum, tickets = _accum_args(pw, x.shape[0], scratch)
-    ext().gemm_tc(pw.data, pw.fmt, pw.n, pw.k, x, out, epi, bias, accum, tickets, ksplit if accum is not None else 1,
+    if tickets is None and scratch is not None and pw.n_tiles <= scratch.tickets.numel():
+        tickets = scratch.tickets          # wider than the split-K accumulator (the LM head): the small-batch kernel needs the counters only
+    ext().gemm_tc(pw.data, pw.fmt, pw.n, pw.k, x, out, epi, bias, accum, tickets, ksplit if tickets is not None else 1,
                   scratch.status if scratch is not None else None, debug_ptr, flags, tp,
                   scratch.partials if scratch is not None else None)
     _count()

@@ -495,7 +495,9 @@ static void gemm_tc(const Tensor& w, int64_t fmt, int64_t n, int64_t k, const Te
     p.out = out.data_ptr(); p.out_stride = (int)out.stride(0); p.out_f32 = out.scalar_type() == torch::kFloat32;
     p.epi = (int)epi; p.bias = cptr<float>(bias); p.status = mptr<int>(status);
     p.accum = mptr<float>(accum); p.tickets = mptr<unsigned>(tickets); p.ksplit = (int)ksplit;
-    if (partials.has_value() && partials->numel() >= 148 * 2 * 128 * 32 && partials->scalar_type() == torch::kFloat32) p.partials = mptr<float>(partials);
+    const int64_t slot_rows = p.m <= 32 ? 32 : (p.m <= 64 ? 64 : 128);              // two slots of [rows][128] for every CTA
+    if (partials.has_value() && partials->numel() >= 148 * 2 * 128 * slot_rows && partials->scalar_type() == torch::kFloat32) p.partials = mptr<float>(partials);
+    if (tickets.has_value() && tickets->numel() < (n + 127) / 128) p.tickets = nullptr;
     p.debug = reinterpret_cast<int*>(debug_ptr); p.flags = (int)flags;
     p.tp = tp.has_value() ? reinterpret_cast<const llm::TpFuse*>(tp->data_ptr()) : nullptr;
     if (tp.has_value()) TORCH_CHECK(p.m <= 32 && epi == llm::EPI_RESID, "fused tensor-parallel epilogue: residual mode, at most 32 rows");

@@ -577,7 +577,7 @@ static cudaError_t launch_one(const GemmTcParams& p, int ksplit, cudaStream_t st
 }  // namespace tc
 
 void gemm_tc_plan(int m, int n, int k, int ksplit_hint, int* block_m, int* ksplit) {
-    const int bm = m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256));     // 32: persistent small-batch kernel
+    const int bm = m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256));     // up to 128: persistent small-batch kernel
     const int tiles = ((n + 127) / 128) * ((m + bm - 1) / bm);
     const int kb = k / 256;
     int ks = ksplit_hint;
@@ -638,7 +638,13 @@ cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st) {
         ks = 1;
     }
     if (ks > 1 && (!p.accum || !p.tickets)) ks = 1;
-    if (bm == 32 && !p.rs_on && p.groups == 0) return launch_gemm_tc_small(p, bm, (p.accum && p.tickets && p.ksplit != 1) ? 0 : 1, st);
+    if (bm <= 128 && !p.rs_on && !p.ag_on && p.groups == 0) {
+        // Up to 128 rows the product is a stream of weights: the persistent kernel reads it once, every SM the same share.  It
+        // wants the chunks on 16-byte boundaries and work indices of 32 bits; calls of 33 rows or more without these keep
+        // the kernel of large tiles, as they always had it.
+        const bool fits = !(reinterpret_cast<uintptr_t>(p.w) & 15) && ((unsigned long long)((p.n + 127) / 128) * (p.k / 256) + 1) * 148ull < (1ull << 32);
+        if (bm == 32 || (fits && !p.tp)) return launch_gemm_tc_small(p, bm, (p.tickets && p.ksplit != 1) ? 0 : 1, st);
+    }
     switch (p.fmt) {
         case FMT_Q4_K: return launch_fmt<FMT_Q4_K>(p, bm, ks, st);
         case FMT_Q5_K: return launch_fmt<FMT_Q5_K>(p, bm, ks, st);

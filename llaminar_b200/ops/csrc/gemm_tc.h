@@ -55,7 +55,7 @@ struct GemmTcParams {
     float* accum;              // split-K scratch fp32 [m_pad][accum_stride], zero between calls
     unsigned* tickets;         // split-K counters [n_tiles * m_tiles], zero between calls
     int accum_stride;
-    float* partials;           // small-batch kernel: [grid][2][32 tokens][128 rows] fp32 slots for split tiles (nullptr: atomics into accum)
+    float* partials;           // small-batch kernel: [grid][2][tokens of a tile][128 rows] fp32 slots for split tiles (nullptr: atomics into accum, or whole tiles)
     int ksplit;                // 0 = automatic
     int* status;               // optional device word: set to STATUS_TIMEOUT if a pipeline wait gave up
     int* debug;                // optional trace buffer (progress markers / ns timestamps written by the kernels); nullptr in production
@@ -79,7 +79,7 @@ struct GemmTcParams {
 };
 
 cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st);
-// small-batch kernel (block_m 32 or 64), implemented in gemm_tc_small.cu
+// small-batch kernel (block_m 32, 64 or 128), implemented in gemm_tc_small.cu
 cudaError_t launch_gemm_tc_small(const GemmTcParams& p, int block_m, int ksplit, cudaStream_t st);
 // tile height the launcher uses for a fused reduce-scatter launch of m rows (the owners' counters are per tile of that height)
 int gemm_tc_rs_block_m(int m, int rows_per_rank);

@@ -1,5 +1,5 @@
-// Small-batch (1 <= M <= 64 rows; the engine uses it for 5..64) variant of the tcgen05 dequant GEMM: the weight-streaming,
-// memory-bound regime of batched decode.  out[M, N] = x[M, K] * dequant(W)[N, K]^T with weights in the MMA M dimension.
+// Small-batch variant of the tcgen05 dequant GEMM, for tiles of 32, 64 or 128 tokens (the engine uses it for 5..128): the
+// weight-streaming regime of batched decode and of short prompts.  out[M, N] = x[M, K] * dequant(W)[N, K]^T with weights in the MMA M dimension.
 //
 // Differences from the large-tile kernel in gemm_tc.cu:
 //   * the packed weight chunks (128 rows x 256 columns, ~14-34 KB) are fetched by one producer warp with 16-byte cp.async
@@ -54,7 +54,8 @@ LLM_DEVICE void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
 
 
 template <int FMT, int BM> struct Cfg {
-    static_assert(BM == 32, "the small-batch kernel is built for one 32-token tile");
+    static_assert(BM == 32 || BM == 64 || BM == 128, "one tile of 32, 64 or 128 tokens");
+    static constexpr bool WIDE = BM > 32;                 // more than 8 tokens per epilogue thread: epilogue in groups of 8
     static constexpr int B_ATOM_BYTES = BM * 128;         // activation tile: BM tokens x 64 columns, 128B-swizzled
     // Formats converted by two alternating sets of eight warps (see TWO_SETS below): each warp set owns one operand set and
     // the raw ring has an even number of slots, so that every waiter meets each of its barriers on EVERY revolution.  A
@@ -62,13 +63,14 @@ template <int FMT, int BM> struct Cfg {
     // then passes on a stale phase (with three operand sets, or five raw slots, the alternating warp sets did exactly
     // that: an "unspecified launch failure" of the Q8_0 kernel on a 10240 x 5120 matrix).
     static constexpr bool TWO_SETS = (FMT == FMT_Q8_0 || FMT == FMT_IQ3_S);
-    static constexpr int N_SETS = TWO_SETS ? 2 : 3;       // chunks in flight between the dequant warps and the MMA issuers
+    // chunks in flight between the dequant warps and the MMA issuers; 128 tokens leave tensor memory for two
+    static constexpr int N_SETS = TWO_SETS || BM == 128 ? 2 : 3;
     static constexpr int N_B_STAGES = 4 * N_SETS;         // per chunk four 64-column activation atoms
     static constexpr int RING_BYTES = N_B_STAGES * B_ATOM_BYTES;
     static constexpr int CHUNK = FmtTraits<FMT>::CHUNK;
     static constexpr int BUDGET = 218 * 1024 - RING_BYTES;
     static constexpr int RAW_SLOTS_ = BUDGET / CHUNK;
-    static constexpr int RAW_SLOTS = (RAW_SLOTS_ > 8 ? 8 : RAW_SLOTS_) & ~1;
+    static constexpr int RAW_SLOTS = TWO_SETS || BM == 32 ? (RAW_SLOTS_ > 8 ? 8 : RAW_SLOTS_) & ~1 : (RAW_SLOTS_ > 8 ? 8 : RAW_SLOTS_);
     static_assert(RAW_SLOTS >= 2, "not enough shared memory for the raw chunk ring");
     static constexpr int SMEM_BYTES = RING_BYTES + RAW_SLOTS * CHUNK + 1024;
     static constexpr int COLS_PER_WARP = BM / 4;          // epilogue: 4 column parts x 4 lane quarters
@@ -87,7 +89,9 @@ template <int FMT, int BM> struct Cfg {
     // sets of eight warps on alternate chunks (measured per-chunk period 1.59 -> 1.16 us and 2.20 -> 1.57 us); the
     // ALU-bound k-quants keep all sixteen warps on one chunk (two sets: 0.91 -> 1.10 us for Q4_K).
     static constexpr int DQ_WARPS_PER_CHUNK = TWO_SETS ? N_DQ_WARPS / 2 : N_DQ_WARPS;
-    static constexpr int N_ISSUERS = 2;
+    // Wider tiles issue from one warp into one accumulator: two of them, double-buffered, would take the operand sets' columns,
+    // and an MMA of 64 or 128 columns occupies the pipe for longer than its issue.
+    static constexpr int N_ISSUERS = WIDE ? 1 : 2;
     static constexpr int ACC_PER_ISSUER = 1;
     static constexpr int ACC_SET_COLS = N_ISSUERS * ACC_PER_ISSUER * BM;
     static constexpr int A_COLS_OFFSET = 2 * ACC_SET_COLS;
@@ -567,6 +571,125 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
             if (warp == 0 && lane == 0) stamp(3, ui_ * 4 + 3);
             return true;
         };
+        // Epilogue of a tile of 64 or 128 tokens: the accumulator goes by in groups of 8 columns, the parked partial sums of the next
+        // group in flight while one is finished.  The protocol of split tiles is the one above (always with slots: without
+        // them the launcher gives every CTA whole tiles).
+        auto epilogue_wide = [&](const Unit& u, int ui_) -> bool {
+            const int buf = ui_ & 1, c0 = part * CW;
+            constexpr int MAX_C = 4;
+            const int c_first = u.contributors > 1 ? it.cta_of(u.tile * k_blocks) : 0;
+            const int c_last = u.contributors > 1 ? it.cta_of(u.tile * k_blocks + k_blocks - 1) : 0;
+            const int nc = c_last - c_first + 1;
+            const bool finisher = u.contributors > 1 && (int)blockIdx.x == c_first;
+            auto slot_of = [&](int c) {
+                const int c_pos = (int)(((unsigned)c * (unsigned)it.total) / (unsigned)it.G);
+                return p.partials + ((size_t)c * 2 + (c_pos / k_blocks == u.tile ? 0 : 1)) * (128 * BM) + row;
+            };
+            float parked[MAX_C - 1][8];
+            auto fetch = [&](int j) {
+#pragma unroll
+                for (int i = 1; i < MAX_C; ++i) {
+                    if (i < nc) {
+                        const float* theirs = slot_of(c_first + i) + (c0 + j * 8) * 128;
+#pragma unroll
+                        for (int t = 0; t < 8; ++t) parked[i - 1][t] = __ldcg(theirs + t * 128);
+                    }
+                }
+            };
+            if (finisher) {
+                const unsigned target = (unsigned)(N_DQ_WARPS * (u.contributors - 1));
+                int got = 1;
+                if (lane == 0) {
+                    got = 0;
+                    for (uint32_t i = 0; i < SPIN_LIMIT; ++i) {
+                        if (ld_acquire_gpu(&p.tickets[u.tile]) >= target) { got = 1; break; }
+                        if (i > 64) { if (abort_flag[0]) break; __nanosleep(32); }
+                    }
+                    if (!got) abort_flag[0] = 1;
+                }
+                got = __shfl_sync(0xffffffffu, got, 0);
+                __syncwarp();
+                if (!got) return false;
+                if (lane == 0) mbar_arrive(tick_bar);           // warp 0 puts the counter back once every warp has seen it (see above)
+                if (warp == 0) {
+                    if (!mbar_wait(tick_bar, tick_syncs & 1, abort_flag)) return false;
+                    if (lane == 0) p.tickets[u.tile] = 0u;
+                }
+                ++tick_syncs;
+                fetch(0);
+            }
+            if (!mbar_wait(accf_bar + buf * 8, (ui_ >> 1) & 1, abort_flag)) return false;
+            tc_fence_after();
+            __syncwarp();
+            const int n_row = u.tile * 128 + row;
+            const float bias = p.bias && n_row < p.n ? p.bias[n_row] : 0.f;
+#pragma unroll 1
+            for (int j = 0; j < CW / 8; ++j) {
+                const int m0 = c0 + j * 8;
+                uint32_t r[8];
+                tmem_ld8(tmem_base + ((uint32_t)(q * 32) << 16) + buf * C::ACC_SET_COLS + m0, r);
+                float v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+                if (u.contributors > 1 && !finisher) {
+                    float* mine = p.partials + ((size_t)blockIdx.x * 2 + (ui_ > 0 ? 1 : 0)) * (128 * BM) + row;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) __stcg(mine + (m0 + i) * 128, v[i]);
+                    continue;
+                }
+                if (finisher) {
+#pragma unroll
+                    for (int c = 1; c < MAX_C; ++c) {
+                        if (c < nc) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) v[i] += parked[c - 1][i];
+                        }
+                    }
+                    for (int c = c_first + MAX_C; c <= c_last; ++c) {
+                        const float* theirs = slot_of(c) + m0 * 128;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[i] += __ldcg(theirs + i * 128);
+                    }
+                    if (j + 1 < CW / 8) fetch(j + 1);
+                }
+                if (p.epi == EPI_SWIGLU) {
+                    // lanes l and l + 16 hold gate and up of one output column: the lower lane finishes the even tokens, the
+                    // upper lane the odd ones
+                    const int col = u.tile * 64 + g * 16 + (lane & 15);
+                    const bool lower = lane < 16;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float other = __shfl_xor_sync(0xffffffffu, lower ? v[2 * i + 1] : v[2 * i], 16);
+                        const float gate = lower ? v[2 * i] : other, up = lower ? other : v[2 * i + 1];
+                        const int m = m0 + 2 * i + (lower ? 0 : 1);
+                        if (m < p.m && col < p.n / 2) static_cast<__nv_bfloat16*>(p.out)[(size_t)m * p.out_stride + col] = __float2bfloat16(silu(gate) * up);
+                    }
+                } else if (n_row < p.n) {
+                    if (p.epi == EPI_RESID) {
+                        float* h = static_cast<float*>(p.out) + (size_t)m0 * p.out_stride + n_row;
+                        float hv[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) hv[i] = (m0 + i < p.m) ? __ldcg(h + (size_t)i * p.out_stride) : 0.f;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (m0 + i < p.m) h[(size_t)i * p.out_stride] = hv[i] + v[i] + bias;
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            if (m0 + i >= p.m) continue;
+                            const size_t idx = (size_t)(m0 + i) * p.out_stride + n_row;
+                            if (p.out_f32) static_cast<float*>(p.out)[idx] = v[i] + bias;
+                            else static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16(v[i] + bias);
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acce_bar + buf * 8);       // accumulator may be overwritten by unit ui + 2
+            if (u.contributors > 1 && !finisher && lane == 0) mbar_arrive(sig_bar);
+            return true;
+        };
         // The epilogue of a unit is run two chunks into the next unit: by then its MMAs have completed, so the dequant warps
         // never sit out the drain of the operand ring, and the issuers work through those two chunks meanwhile.
         constexpr int DEFER = 2;
@@ -575,7 +698,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
         auto flush = [&]() -> bool {
             if (p_ui < 0) return true;
             publish();
-            const bool r = epilogue(pu, p_ui, p_cc0);
+            bool r;
+            if constexpr (C::WIDE) r = epilogue_wide(pu, p_ui);
+            else r = epilogue(pu, p_ui, p_cc0);
             p_ui = -1;
             return r;
         };
@@ -637,6 +762,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
                     sink.emit64(rs.o);
                     pend_set = set;
                     pend_slot = slot;
+                    // with two operand sets the next chunk waits for the MMAs of the chunk before this one: a late publication
+                    // would put conversion and MMAs in turn (51200 x 5120 Q4_K, 128 rows: 78 us late, 63 us at once)
+                    if constexpr (C::N_SETS == 2) publish();
                 }
                 // The alternating warp sets publish at once: a set owns one operand set, so its next chunk's operand set frees
                 // only after this chunk has been published and multiplied.
@@ -713,7 +841,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
     } else {
         // ---------------- MMA issuers: warp w takes the chunks of parity w ----------------
         const int w = warp - (N_DQ_WARPS + 2);
-        if (elect_one()) {
+        if (w < C::N_ISSUERS && elect_one()) {
             constexpr uint32_t idesc = instr_desc(BM);
             int cc = 0, ui = 0;
             bool ok = true;
@@ -732,8 +860,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
                     const uint32_t acc_base = tmem_base + buf * C::ACC_SET_COLS + w * C::ACC_PER_ISSUER * BM;
                     const uint32_t a_tmem = tmem_base + C::A_COLS_OFFSET + set * C::A_CHUNK_COLS;
 #pragma unroll
-                    for (int a2 = 0; a2 < 2; ++a2) {
-                        const int a = 2 * w + a2;
+                    for (int a2 = 0; a2 < 4 / C::N_ISSUERS; ++a2) {
+                        const int a = (4 / C::N_ISSUERS) * w + a2;
                         const uint64_t bdesc = smem_desc_sw128(smem_base + (set * 4 + a) * C::B_ATOM_BYTES);
 #pragma unroll
                         for (int k4 = 0; k4 < 4; ++k4)      // 16 columns of K = 8 TMEM columns of A, 32 bytes of the swizzled B row
@@ -805,7 +933,8 @@ static cudaError_t launch_one(const GemmTcParams& p, int ksplit, cudaStream_t st
     GemmTcParams q = p;
     const int n_tiles = (p.n + 127) / 128, k_blocks = p.k / 256;
     if ((unsigned long long)(n_tiles * (long long)k_blocks + 1) * 148ull >= (1ull << 32)) return cudaErrorInvalidValue;   // 32-bit work indices
-    const bool streamk = ksplit != 1 && p.accum && p.tickets;
+    // split tiles need the slot workspace; the 32-token form can do with atomics into `accum` instead
+    const bool streamk = ksplit != 1 && p.tickets && (p.partials || (p.accum && !C::WIDE));
     q.flags = (p.flags & ~2) | (streamk ? 2 : 0);
     const int units = streamk ? n_tiles * k_blocks : n_tiles;
     static int cached_sms = 0;
@@ -820,13 +949,19 @@ static cudaError_t launch_one(const GemmTcParams& p, int ksplit, cudaStream_t st
         if (g < 1) g = 1;
         if (g < grid) grid = g;
     }
-    if (grid > 148) q.partials = nullptr;            // the slot workspace is sized for 148 CTAs
+    if (grid > 148) {                                // the slot workspace is sized for 148 CTAs
+        if (C::WIDE) grid = 148; else q.partials = nullptr;
+    }
     return launch_pdl(gemm_tc_small_kernel<FMT, BM>, dim3(grid), dim3(THREADS), C::SMEM_BYTES, st, tmap, q);
 }
 
 template <int FMT>
 static cudaError_t launch_fmt(const GemmTcParams& p, int bm, int ks, cudaStream_t st) {
-    if (bm == 32) return launch_one<FMT, 32>(p, ks, st);
+    switch (bm) {
+        case 32: return launch_one<FMT, 32>(p, ks, st);
+        case 64: return launch_one<FMT, 64>(p, ks, st);
+        case 128: return launch_one<FMT, 128>(p, ks, st);
+    }
     return cudaErrorInvalidValue;
 }
 
