@@ -256,9 +256,9 @@ def attn_decode(q, kv, out, block_table, seq_lens, n_heads, n_kv_heads, head_dim
 def attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, head_dim, scale, max_q_len,
                  tensor_core: bool | None = None, scratch: "Scratch | None" = None) -> None:
     """Causal GQA attention of a prefill chunk over the paged cache.  ``tensor_core`` picks the tcgen05 kernel (head_dim 128),
-    otherwise the mma.sync kernel runs.  Default: the tcgen05 kernel for chunks of at least ATTN_TC_MIN_ROWS query rows per
-    sequence (measured 283 vs 246 TFLOP/s at 2048 rows, 323 vs 234 at 4096, but 223 vs 237 at 1024, where its per-CTA
-    start-up weighs more); LLAMINAR_ATTN_TC=0 turns it off."""
+    otherwise the mma.sync kernel runs.  Default: the tcgen05 kernel wherever it fits; it is the faster one from ATTN_TC_MIN_ROWS
+    query rows on (32 / 8 heads: 8.9 vs 11.3 us at 16 rows, 23.6 vs 82.6 at 1024, 164 vs 785 at 4096, 120 vs 414 at 500 rows
+    behind 7000 tokens); LLAMINAR_ATTN_TC=0 turns it off."""
     if tensor_core is None:
         tensor_core = head_dim == 128 and max_q_len >= ATTN_TC_MIN_ROWS and _attn_tc_default()
     status = scratch.status if (tensor_core and scratch is not None) else None
@@ -286,7 +286,7 @@ def gdn_step(inp: torch.Tensor, C: int, z_off: int, ab_off: int, conv_w: torch.T
     _count(2)
 
 
-ATTN_TC_MIN_ROWS = 1536
+ATTN_TC_MIN_ROWS = 1
 _ATTN_TC = None
 
 

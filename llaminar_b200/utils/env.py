@@ -34,7 +34,7 @@ REGISTRY: tuple[EnvVar, ...] = (
     EnvVar("LLAMINAR_SKIP_ALLREDUCE", bool, False, "debug: skip tensor-parallel all-reduces (results are wrong; isolates compute time)"),
     EnvVar("LLAMINAR_VALIDATE_TENSORS", bool, False, "check every index of a step's inputs on the host before launch; scan activations for NaN/Inf after every layer"),
     EnvVar("LLAMINAR_PDL", bool, True, "launch the decode-path kernels with programmatic dependent launch (prologues overlap the previous kernel)"),
-    EnvVar("LLAMINAR_ATTN_TC", bool, True, "long prefill chunks (head_dim 128) run attention on the tcgen05 kernel instead of the mma.sync kernel"),
+    EnvVar("LLAMINAR_ATTN_TC", bool, True, "prefill chunks (head_dim 128) run attention on the tcgen05 kernel instead of the mma.sync kernel"),
     EnvVar("LLAMINAR_TUNING_FILE", str, "", "JSON table of measured kernel launch parameters (written by python -m llaminar_b200.ops.tuning)"),
     EnvVar("LLAMINAR_NO_CUDA_GRAPHS", bool, False, "run decode steps eagerly instead of replaying CUDA graphs"),
     EnvVar("LLAMINAR_HEARTBEAT_S", float, 2.0, "interval of the per-rank heartbeat"),

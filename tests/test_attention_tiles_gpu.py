@@ -1,0 +1,82 @@
+"""The tcgen05 prefill attention at the edges of its tiles: 128 query rows and 128 keys, two slots (heads of a group, or query tiles
+where the group is odd) per CTA."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+# P is rounded to bf16 (2^-9 of each term at most, zero mean), the output once more; the sums are fp32
+REL = 6e-3
+
+
+def _reference(q, k, v, ctx, window=0, softcap=0.0, sink=None):
+    """q [L, H, D] behind ctx keys, k / v [ctx + L, Hk, D]; 64-bit."""
+    L, H, D = q.shape
+    k, v = (x.double().repeat_interleave(H // x.shape[1], 1) for x in (k, v))
+    s = torch.einsum("lhd,shd->hls", q.double(), k) / math.sqrt(D)
+    if softcap:
+        s = softcap * torch.tanh(s / softcap)
+    row, col = torch.arange(L, device=DEV)[:, None] + ctx, torch.arange(ctx + L, device=DEV)[None]
+    s = s.masked_fill((col > row) | (window > 0) & (col <= row - window), -math.inf)
+    if sink is not None:
+        s = torch.cat([s, sink.double()[:, None, None].expand(H, L, 1)], 2)
+        v = torch.cat([v, torch.zeros_like(v[:1])])
+    return torch.einsum("hls,shd->lhd", torch.softmax(s, -1), v)
+
+
+def _case(heads, kv_heads, lens, ctx, rising, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    D, B = 128, len(lens)
+    pages = max((c + n + 63) // 64 for c, n in zip(ctx, lens)) + 1
+    table = torch.randperm(B * pages, generator=torch.Generator().manual_seed(seed)).view(B, pages).to(torch.int32).to(DEV)
+    kv = torch.zeros(B * pages, 2, kv_heads, 64, D, dtype=torch.bfloat16, device=DEV)
+    q = torch.randn(sum(lens), heads, D, device=DEV, generator=g)
+    if rising:
+        q[..., 0] = 4.0                                          # scores grow with the key's place: the running maximum rises tile by tile
+    q, keys, values = q.bfloat16(), [], []
+    for b, (c, n) in enumerate(zip(ctx, lens)):
+        k, v = torch.randn(2, c + n, kv_heads, D, device=DEV, generator=g).bfloat16()
+        if rising:
+            k[..., 0] = (torch.arange(c + n, device=DEV) * 0.05)[:, None]
+        keys.append(k)
+        values.append(v)
+        for t in range(0, c + n, 64):
+            part = slice(t, min(t + 64, c + n))
+            for i, x in enumerate((k, v)):
+                kv[table[b, t // 64], i, :, :part.stop - t] = x[part].transpose(0, 1)
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    return q, kv, table, cu, torch.tensor(ctx, dtype=torch.int32, device=DEV), keys, values
+
+
+def _check(out, q, cu, ctx, keys, values, **how):
+    for b, (k, v) in enumerate(zip(keys, values)):
+        rows = slice(int(cu[b]), int(cu[b + 1]))
+        want = _reference(q[rows], k, v, int(ctx[b]), **how)
+        assert (out[rows].double() - want).norm() <= REL * want.norm(), b
+
+
+@pytest.mark.parametrize("rising", [False, True])
+@pytest.mark.parametrize("heads,kv_heads,lens,ctx", [
+    (8, 2, [1, 127, 128], [0, 0, 0]), (8, 2, [129, 257], [63, 0]), (7, 1, [130, 3, 385], [0, 128, 1]), (14, 2, [255, 64], [1000, 65]),
+    (3, 3, [129, 300], [0, 127]), (1, 1, [1], [0]), (16, 1, [17], [2500]), (28, 4, [37], [0])])
+def test_tiles(heads, kv_heads, lens, ctx, rising):
+    from llaminar_b200 import ops
+    q, kv, table, cu, c, keys, values = _case(heads, kv_heads, lens, ctx, rising)
+    out, sc = torch.full_like(q, float("nan")), ops.scratch_for(DEV)
+    ops.attn_prefill(q, kv, out, table, cu, c, heads, kv_heads, 128, 1 / math.sqrt(128), max(lens), tensor_core=True, scratch=sc)
+    assert int(sc.status[0]) == 0
+    _check(out, q, cu, c, keys, values)
+
+
+@pytest.mark.parametrize("window,softcap,sink", [(1, 0.0, False), (100, 0.0, True), (129, 20.0, False), (0, 30.0, True)])
+def test_masks(window, softcap, sink):
+    from llaminar_b200.ops import grouped
+    heads, kv_heads, lens, ctx = 7, 1, [140, 300], [200, 0]
+    q, kv, table, cu, c, keys, values = _case(heads, kv_heads, lens, ctx, False, 1)
+    logits = torch.randn(heads, device=DEV) if sink else None
+    out, status = torch.full_like(q, float("nan")), torch.zeros(4, dtype=torch.int32, device=DEV)
+    grouped.attn_prefill(q, kv, out, table, cu, c, 1 / math.sqrt(128), max(lens), window, logits, None, status, softcap=softcap)
+    assert int(status[0]) == 0
+    _check(out, q, cu, c, keys, values, window=window, softcap=softcap, sink=logits)
