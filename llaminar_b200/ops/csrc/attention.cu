@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(128) paged_attn_decode_kernel(const AttnDecode
     // thread t handles column t % D of rows t / D, t / D + 128 / D, ...
     const int col = threadIdx.x % D;
     // quotient of one output value: the sink's share of the denominator, the output gate
-    auto store = [&](int i, float m, float l, float acc) {
+    auto store = [&](int i, int col, float m, float l, float acc) {
         const int r = i / G, head = kvh * G + i % G;
         const size_t row = (size_t)seq * R + r;
         if (p.sink) l += exp2f(p.sink[head] * 1.4426950408889634f - m);
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(128) paged_attn_decode_kernel(const AttnDecode
             acc += c * s_o[(w * 16 + i) * D + col];
         }
         if (gridDim.y == 1) {
-            store(i, m, l, acc);
+            store(i, col, m, l, acc);
         } else {
             p.part_o[(part_base + i) * D + col] = acc;
             if (col == 0) { p.part_ml[(part_base + i) * 2] = m; p.part_ml[(part_base + i) * 2 + 1] = l; }
@@ -364,29 +364,78 @@ __global__ void __launch_bounds__(128) paged_attn_decode_kernel(const AttnDecode
     if (gridDim.y == 1) return;
 
     // ---- last CTA of this (sequence, kv head) merges the splits ----
+    // Two round trips to L2 whatever the number of rows and splits: the maxima and sums of all (row, split) pairs at once, then the
+    // partial outputs, a warp per row with eight splits in flight (32 / 8 heads, one sequence of 700 tokens in 6 splits: 7.7 us
+    // against 14.2 for rows one after the other; three of 6000 tokens, 8-bit, 13 splits: 20.8 against 36.1).
     __shared__ int s_last;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned t = atomicAdd(&p.tickets[seq * p.n_kv_heads + kvh], 1u);
+        unsigned t;      // releases this CTA's partials (every thread's, through the barrier) and acquires the others'
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(t) : "l"(&p.tickets[seq * p.n_kv_heads + kvh]) : "memory");
         s_last = (t == gridDim.y - 1);
         if (s_last) p.tickets[seq * p.n_kv_heads + kvh] = 0u;
     }
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
-    const size_t pb = (((size_t)seq * p.n_kv_heads + kvh) * gridDim.y) * 16;
-    for (int i = threadIdx.x / D; i < rows; i += 128 / D) {
-        float m = -INFINITY;
-        for (int s = 0; s < (int)gridDim.y; ++s) m = fmaxf(m, __ldcg(&p.part_ml[(pb + s * 16 + i) * 2]));
-        float l = 0.f, acc = 0.f;
-        for (int s = 0; s < (int)gridDim.y; ++s) {
-            const float ms = __ldcg(&p.part_ml[(pb + s * 16 + i) * 2]);
-            const float c = ms == -INFINITY ? 0.f : exp2f(ms - m);
-            l += c * __ldcg(&p.part_ml[(pb + s * 16 + i) * 2 + 1]);
-            acc += c * __ldcg(&p.part_o[(pb + s * 16 + i) * D + col]);
+    const int S = (int)gridDim.y;
+    const size_t pb = (((size_t)seq * p.n_kv_heads + kvh) * S) * 16;
+    constexpr int BLOCK = 64, TPR = 32, STEP = 128 / TPR, RPT = 16 / STEP, CPT = D / TPR;      // 32 threads per row, up to four rows each
+    static_assert(16 * BLOCK * 2 * 4 <= DecodeSmem<D, Q8>::BYTES, "maxima and sums of a block of splits");
+    float* s_w = reinterpret_cast<float*>(smem);             // [rows][BLOCK][2]: maximum and sum
+    float m[RPT], l[RPT], acc[RPT][CPT];
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        m[r] = -INFINITY; l[r] = 0.f;
+#pragma unroll
+        for (int e = 0; e < CPT; ++e) acc[r][e] = 0.f;
+    }
+    for (int b0 = 0; b0 < S; b0 += BLOCK) {
+        const int n = min(BLOCK, S - b0);
+        __syncthreads();
+        for (int j = threadIdx.x; j < rows * n; j += 128) {
+            const int i = j / n, sp = j - i * n;
+            const float* ml = p.part_ml + (pb + (size_t)(b0 + sp) * 16 + i) * 2;
+            const float pm = __ldcg(ml), pl = __ldcg(ml + 1);
+            s_w[(i * BLOCK + sp) * 2] = pm;
+            s_w[(i * BLOCK + sp) * 2 + 1] = pl;
         }
-        store(i, m, l, acc);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) {
+            const int i = warp + r * STEP;
+            if (i >= rows) break;
+            const float* w = s_w + i * BLOCK * 2;
+            float mn = m[r];
+            for (int sp = 0; sp < n; ++sp) mn = fmaxf(mn, w[2 * sp]);
+            const float old = m[r] == -INFINITY ? 0.f : exp2f(m[r] - mn);
+            m[r] = mn;
+            l[r] *= old;
+#pragma unroll
+            for (int e = 0; e < CPT; ++e) acc[r][e] *= old;
+            const float* part = p.part_o + (pb + (size_t)b0 * 16 + i) * D + lane;
+            for (int s0 = 0; s0 < n; s0 += 8) {
+                float v[8][CPT];
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+#pragma unroll
+                    for (int e = 0; e < CPT; ++e) v[k][e] = s0 + k < n ? __ldcg(part + (size_t)(s0 + k) * 16 * D + e * TPR) : 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    if (s0 + k >= n) break;
+                    const float c = w[2 * (s0 + k)] == -INFINITY ? 0.f : exp2f(w[2 * (s0 + k)] - mn);
+                    l[r] += c * w[2 * (s0 + k) + 1];
+#pragma unroll
+                    for (int e = 0; e < CPT; ++e) acc[r][e] += c * v[k][e];
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+        const int i = warp + r * STEP;
+        if (i >= rows) break;
+#pragma unroll
+        for (int e = 0; e < CPT; ++e) store(i, lane + e * TPR, m[r], l[r], acc[r][e]);
     }
 }
 
