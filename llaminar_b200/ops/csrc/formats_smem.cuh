@@ -264,6 +264,10 @@ struct DequantAtomQ4KRt {
         const uint32_t qaddr = raw + T::P_QS + ((uint32_t)(g * 8 + 2 * A) << 9) + ((uint32_t)lane << 4);
         r.q0 = lds_v4(qaddr);
         r.q1 = lds_v4(qaddr + 512);
+        scales(meta, A, r);
+        return r;
+    }
+    LLM_DEVICE static void scales(const uint4& meta, int A, Regs& r) {
         // 6-bit scales / minima of sub-blocks 2A and 2A + 1: bytes (2A & 3) and (2A & 3) + 1 of the three packed words
         const int sh = (A & 1) << 4;
         const uint32_t a2 = meta.y >> sh, b2 = meta.z >> sh, c2 = meta.w >> sh;
@@ -283,7 +287,6 @@ struct DequantAtomQ4KRt {
         r.s_hi = __float2bfloat162_rn(fminf(fmaf(sc_hi, d100, d100c) * k29, BIG));
         r.b_lo = __float2bfloat162_rn(fmaf(mn_lo, ndmin, ndminc));
         r.b_hi = __float2bfloat162_rn(fmaf(mn_hi, ndmin, ndminc));
-        return r;
     }
     // all 64 values (32 packed pairs) of the atom into `o`, which the caller then hands to one tensor-memory store
     LLM_DEVICE static void convert(const Regs& r, uint32_t (&o)[32]) {

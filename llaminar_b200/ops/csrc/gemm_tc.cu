@@ -645,6 +645,15 @@ cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st) {
         const bool fits = !(reinterpret_cast<uintptr_t>(p.w) & 15) && ((unsigned long long)((p.n + 127) / 128) * (p.k / 256) + 1) * 148ull < (1ull << 32);
         if (bm == 32 || (fits && !p.tp)) return launch_gemm_tc_small(p, bm, (p.tickets && p.ksplit != 1) ? 0 : 1, st);
     }
+    // More rows, and the groups of expert GEMMs, run on pairs of CTAs; the kernel here keeps the fused collectives, forced splits, traces
+    // and more groups than the pairs keep offsets for.
+    if (!p.rs_on && !p.ag_on && !p.debug && p.groups <= 256) {
+        if (p.groups > 0) return launch_gemm_tc_pair(p, bm, st);
+        // (up to 256 rows of a narrow and long matrix leave most pairs without a tile: there this kernel splits K instead.
+        // 5120 x 25600 Q4_K, 160 rows: 99 us here, 124 us there; 4096 x 12288: 62 and 63 us.)
+        const bool narrow = ks > 1 && p.k >= 64 * 256 && (p.n + 127) / 128 * ((p.m + 255) / 256) <= 74;
+        if (bm == 256 && p.ksplit <= 1 && !narrow) return launch_gemm_tc_pair(p, gemm_pair_tokens(p.fmt, p.m, p.n, p.k), st);
+    }
     switch (p.fmt) {
         case FMT_Q4_K: return launch_fmt<FMT_Q4_K>(p, bm, ks, st);
         case FMT_Q5_K: return launch_fmt<FMT_Q5_K>(p, bm, ks, st);

@@ -81,6 +81,9 @@ struct GemmTcParams {
 cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st);
 // small-batch kernel (block_m 32, 64 or 128), implemented in gemm_tc_small.cu
 cudaError_t launch_gemm_tc_small(const GemmTcParams& p, int block_m, int ksplit, cudaStream_t st);
+// persistent kernel of CTA pairs for many rows and for the grouped mode (gemm_tc_pair.cu); `tokens`: rows of a tile, a multiple of 32 up to 256
+cudaError_t launch_gemm_tc_pair(const GemmTcParams& p, int tokens, cudaStream_t st);
+int gemm_pair_tokens(int fmt, int m, int n, int k);
 // tile height the launcher uses for a fused reduce-scatter launch of m rows (the owners' counters are per tile of that height)
 int gemm_tc_rs_block_m(int m, int rows_per_rank);
 // tokens per CTA tile and split factor the launcher would use (for sizing scratch)
