@@ -200,10 +200,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
     __syncthreads();
     tc_fence_after();
     // Everything above touched only this CTA's shared and tensor memory.  The weights are constants, so the raw-chunk producer
-    // starts filling its ring at once (under programmatic dependent launch that overlaps the tail of the previous kernel) and
-    // joins the wait only before its first wait on a ring slot; every other role waits here, before it reads activations or
-    // writes outputs and scratch.
-    if (warp != N_DQ_WARPS) pdl_wait();
+    // starts filling its ring at once (under programmatic dependent launch that overlaps the tail of the previous kernel) and the
+    // dequant warps fill the operand sets; they join the wait before their first wait on a ring slot or an operand set, and before
+    // an epilogue.  The other roles wait here, before they read activations.  (With the dequant warps waiting here as well a layer of
+    // the 8B shape took 121 us at 32 rows instead of 115, the two launches of its query, key and value matrices 24.3 instead of 20.8.)
+    if (warp > N_DQ_WARPS) pdl_wait();
     const uint32_t tmem_base = s_tmem;
     volatile int* abort_flag = s_abort;
     // optional timeline trace of CTA (flags >> 8): p.debug[role * 1024 + slot] = low 32 bits of the ns timer
@@ -241,7 +242,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
         constexpr int CW = C::COLS_PER_WARP;
         TmemSink sink{0};
         int cc = 0, ui = 0, epi_syncs = 0, tick_syncs = 0;
-        bool ok = true;
+        bool ok = true, joined = false;
+        auto join = [&]() { if (!joined) { pdl_wait(); joined = true; } };
         // A chunk is published to the MMA issuers one step late (see the conversion loop): pend_* name the chunk that is owed.
         int pend_set = -1, pend_slot = -1;
         auto publish = [&]() {
@@ -698,6 +700,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
         auto flush = [&]() -> bool {
             if (p_ui < 0) return true;
             publish();
+            join();
             bool r;
             if constexpr (C::WIDE) r = epilogue_wide(pu, p_ui);
             else r = epilogue(pu, p_ui, p_cc0);
@@ -710,6 +713,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
                 if (C::TWO_SETS && (cc & 1) != ws) continue;
                 const int slot = cc % R, rphase = (cc / R) & 1;
                 const int set = set_of(cc);
+                if (cc >= C::N_SETS) join();          // from here on an operand set has to be multiplied before it comes free
                 ok = mbar_wait_warp(rawf_bar + slot * 8, rphase, abort_flag);
                 if (LLM_TRACE && warp == 0 && lane == 0) stamp(0, cc * 4 + 0);
                 // Q4_K: the packed bytes and the prepared scales go into registers now, so that the loads and the scale
