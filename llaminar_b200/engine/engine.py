@@ -271,7 +271,8 @@ class LLMEngine:
         words = self._status_words()
         for i, w in enumerate(words):
             self._health_host[i:i + 1].copy_(w[:1], non_blocking=True)
-        self._health_host[7:8].copy_(self._group_failed(words), non_blocking=True)
+        if getattr(self.tp, "size", 1) > 1:             # alone, this rank's own words say it all
+            self._health_host[7:8].copy_(self._group_failed(words), non_blocking=True)
         self._health_queued = True
 
     def _group_failed(self, words: list[torch.Tensor]) -> torch.Tensor:
@@ -651,24 +652,35 @@ class LLMEngine:
     def _forward_chunks(self, chunks: list[tuple[Request, int, list[int]]], logit_rows: list[int]):
         """One forward call over portions of several sequences: (request, first position, tokens), packed in that order.
         Returns (logits of `logit_rows` or None, hidden rows, the batch)."""
-        dev = self.device
-        toks, pos, sid, cu, ctx = [], [], [], [0], []
-        for b, (r, start, tokens) in enumerate(chunks):
-            n = len(tokens)
-            toks.extend(tokens)
-            pos.extend(range(start, start + n))
-            sid.extend([b] * n)
-            cu.append(cu[-1] + n)
+        import numpy as np
+        cu, ctx = [0], []
+        for r, start, tokens in chunks:
+            cu.append(cu[-1] + len(tokens))
             ctx.append(start)
-        bt = torch.zeros(len(chunks), max(len(r.kv.pages) for r, _, _ in chunks), dtype=torch.int32)
-        for i, (r, _, _) in enumerate(chunks):
-            bt[i, :len(r.kv.pages)] = torch.tensor(r.kv.pages, dtype=torch.int32)
-        it = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
-        fb = ForwardBatch(tokens=it(toks), positions=it(pos), seq_ids=it(sid), block_table=bt.to(dev), cu_q=it(cu),
-                          ctx_lens=it(ctx), max_q_len=max(cu[i + 1] - cu[i] for i in range(len(ctx))),
-                          max_kv_len=max(ctx[i] + cu[i + 1] - cu[i] for i in range(len(ctx))), host_cu=cu, host_ctx=ctx,
-                          logit_rows=it(logit_rows) if logit_rows else None,
-                          state_slots=it([r.slot for r, _, _ in chunks]) if self.kv.hybrid is not None else None)
+        T, B, P = cu[-1], len(chunks), max(len(r.kv.pages) for r, _, _ in chunks)
+        # one upload for all index arrays of the step (a list per array, each with its own copy, was 1.5 ms for 8160 tokens)
+        sizes = {"tokens": T, "positions": T, "seq_ids": T, "table": B * P, "cu": B + 1, "ctx": B, "rows": len(logit_rows), "slots": B}
+        at, total = {}, 0
+        for name, n in sizes.items():
+            at[name] = slice(total, total + n)
+            total += (n + 63) & ~63
+        host = np.zeros(total, dtype=np.int32)
+        table = host[at["table"]].reshape(B, P)
+        for b, (r, start, tokens) in enumerate(chunks):
+            lo, hi = cu[b], cu[b + 1]
+            host[lo:hi] = tokens
+            host[at["positions"]][lo:hi] = np.arange(start, start + hi - lo, dtype=np.int32)
+            host[at["seq_ids"]][lo:hi] = b
+            table[b, :len(r.kv.pages)] = r.kv.pages
+        host[at["cu"]], host[at["ctx"]], host[at["rows"]] = cu, ctx, logit_rows
+        if self.kv.hybrid is not None:
+            host[at["slots"]] = [r.slot for r, _, _ in chunks]
+        dev = torch.from_numpy(host).to(self.device)
+        fb = ForwardBatch(tokens=dev[at["tokens"]], positions=dev[at["positions"]], seq_ids=dev[at["seq_ids"]], block_table=dev[at["table"]].view(B, P),
+                          cu_q=dev[at["cu"]], ctx_lens=dev[at["ctx"]], max_q_len=max(cu[i + 1] - cu[i] for i in range(B)),
+                          max_kv_len=max(ctx[i] + cu[i + 1] - cu[i] for i in range(B)), host_cu=cu, host_ctx=ctx,
+                          logit_rows=dev[at["rows"]] if logit_rows else None,
+                          state_slots=dev[at["slots"]] if self.kv.hybrid is not None else None)
         logits, h = self.model.forward(fb, self.kv, want_logits=bool(logit_rows))
         return logits, h, fb
 
@@ -693,7 +705,7 @@ class LLMEngine:
         wanted rows [n, vocab] in the order of the entries, or None when nothing is wanted."""
         V = self._vocab
         for r, tokens, want in entries:
-            if not tokens or any(not 0 <= t < V for t in tokens) or any(not 0 <= w < len(tokens) for w in want):
+            if not tokens or not (0 <= min(tokens) and max(tokens) < V) or any(not 0 <= w < len(tokens) for w in want):
                 raise ValueError("an entry needs tokens of the vocabulary, and wanted places among them")
             if r.kv.length + len(tokens) > self.max_context:
                 raise ValueError(f"sequence of {r.kv.length + len(tokens)} tokens exceeds the context window of {self.max_context}")
@@ -708,7 +720,10 @@ class LLMEngine:
                 r.output.extend(tokens)
             logits = self._decode_logits([r for r, _, _ in entries])
             picked = [i for i, (_, _, want) in enumerate(entries) for _ in want]
-            out = logits[torch.tensor(picked, dtype=torch.long, device=logits.device)] if picked else None
+            if picked == list(range(len(entries))):
+                out = logits.clone()                            # the captured step's own buffer: the next one writes there
+            else:
+                out = logits[torch.tensor(picked, dtype=torch.long, device=logits.device)] if picked else None
         else:
             at, picked = 0, []
             for r, tokens, want in entries:
@@ -719,11 +734,13 @@ class LLMEngine:
                 r.output.extend(tokens)
         for r, tokens, _ in entries:
             r.kv.length += len(tokens)
-        self.check_health()
+        self._queue_health()
+        self.check_health()                                     # the step's one synchronisation
         return self._gather_vocab(out) if out is not None else None
 
     def _decode_logits(self, reqs: list[Request]) -> torch.Tensor:
-        """Logits of one decode step (the last token of every request is the step's input), without sampling."""
+        """Logits of one decode step (the last token of every request is the step's input), without sampling.  The caller
+        synchronises before the next step: until then the staging buffers and the logits are the step's."""
         bucket = next((b for b in BUCKETS if b >= len(reqs)), len(reqs))
         if not self.use_graphs or bucket > self._bmax:
             return self.model.forward(self._decode_batch_tensors(reqs), self.kv)[0]
@@ -735,7 +752,6 @@ class LLMEngine:
             g = self._graphs[(bucket, "logits")] = self._capture_decode(bucket, True, v, sample=False)
         g.replay()
         self.stats["graph_replays"] += 1
-        torch.cuda.current_stream(self.device).synchronize()       # the staging buffers are free for the next step
         return self._logits[:len(reqs)]
 
     def _prefill(self, batch: list[Request]) -> list[StepOutput]:
