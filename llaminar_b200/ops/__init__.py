@@ -143,6 +143,13 @@ def moe_route_only(h, norm_w, eps, router, top_k, renorm, ids, wts, xn_out=None)
     _count()
 
 
+def moe_sort(ids, wts, e0: int, n_local: int, bm: int, pos, row_off, tile_off, xn, xg) -> None:
+    """(token, slot) pairs in the order of the local experts: pos [T, k] and the rows xg[pos] = xn[token]; row_off / tile_off
+    [n_local + 1] are the experts' first rows and first tiles of ``bm`` rows.  Weights of other experts' pairs become 0."""
+    ext().moe_sort(ids, wts, e0, n_local, bm, pos, row_off, tile_off, xn, xg)
+    _count(2)
+
+
 def moe_combine_sorted(h, y, pos, wts, top_k: int) -> None:
     """h[t] += sum_s wts[t, s] * y[pos[t, s]] (slot order; zero-weight slots skipped)."""
     ext().moe_combine_sorted(h, y, pos, wts, top_k)

@@ -111,6 +111,20 @@ static void moe_route_only(const Tensor& h, const Tensor& norm_w, double eps, co
     LLM_CUDA_CHECK(llm::launch_moe_route(p, cur_stream()));
 }
 
+// (token, slot) pairs in expert order and their rows: `wts` of other ranks' experts become 0
+static void moe_sort(const Tensor& ids, Tensor wts, int64_t e0, int64_t n_local, int64_t bm, Tensor pos, Tensor row_off, Tensor tile_off, const Tensor& xn, Tensor xg) {
+    check_cuda(ids, "ids"); check_cuda(xn, "xn"); check_cuda(xg, "xg");
+    const c10::cuda::CUDAGuard guard(ids.device());
+    TORCH_CHECK(ids.scalar_type() == torch::kInt32 && pos.scalar_type() == torch::kInt32 && row_off.scalar_type() == torch::kInt32 && tile_off.scalar_type() == torch::kInt32);
+    TORCH_CHECK(wts.scalar_type() == torch::kFloat32 && xn.scalar_type() == torch::kBFloat16 && xg.scalar_type() == torch::kBFloat16);
+    TORCH_CHECK(ids.dim() == 2 && ids.is_contiguous() && wts.is_contiguous() && pos.is_contiguous() && xn.is_contiguous() && xg.is_contiguous());
+    const int64_t T = ids.size(0), k = ids.size(1), d = xn.size(1);
+    TORCH_CHECK(wts.numel() == T * k && pos.numel() == T * k && row_off.numel() > n_local && tile_off.numel() > n_local && xn.size(0) >= T && xg.size(0) >= T * k && xg.size(1) == d);
+    LLM_CUDA_CHECK(llm::launch_moe_sort(static_cast<const int*>(ids.data_ptr()), static_cast<float*>(wts.data_ptr()), (int)T, (int)k, (int)e0, (int)n_local, (int)bm,
+                                        static_cast<int*>(pos.data_ptr()), static_cast<int*>(row_off.data_ptr()), static_cast<int*>(tile_off.data_ptr()),
+                                        static_cast<const __nv_bfloat16*>(xn.data_ptr()), (int)d, static_cast<__nv_bfloat16*>(xg.data_ptr()), cur_stream()));
+}
+
 static void moe_combine_sorted(Tensor h, const Tensor& y, const Tensor& pos, const Tensor& wts, int64_t top_k) {
     check_cuda(h, "h"); check_cuda(y, "y");
     const c10::cuda::CUDAGuard guard(h.device());
@@ -602,6 +616,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("moe_route", &moe_route);
     m.def("moe_gemv", &moe_gemv);
     m.def("moe_route_only", &moe_route_only);
+    m.def("moe_sort", &moe_sort);
     m.def("moe_combine_sorted", &moe_combine_sorted);
     m.def("gemm_tc_grouped", &gemm_tc_grouped);
     m.def("gemm_tc", &gemm_tc);

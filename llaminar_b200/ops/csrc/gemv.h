@@ -85,6 +85,9 @@ struct MoeRouteParams {
 cudaError_t launch_moe_combine_sorted(float* h, int h_stride, const float* y, const int* pos, const float* wts, int tokens, int top_k, int d,
                                       cudaStream_t st);
 cudaError_t launch_moe_route(const MoeRouteParams& p, cudaStream_t st);
+// Rows of a prompt in expert order (moe_ep.cu): pos [tokens, top_k], row_off and tile_off [n_local + 1], xg [tokens * top_k, d]
+cudaError_t launch_moe_sort(const int* ids, float* wts, int tokens, int top_k, int e0, int n_local, int bm, int* pos, int* row_off, int* tile_off,
+                            const __nv_bfloat16* xn, int d, __nv_bfloat16* xg, cudaStream_t st);
 
 cudaError_t launch_dequant(int fmt, const uint8_t* w, int n, int k, __nv_bfloat16* out, cudaStream_t st);
 cudaError_t launch_gather_rows(int fmt, const uint8_t* w, int k, const int* rows, int n_rows, float* out_f32,
