@@ -166,28 +166,30 @@ def gemm_grouped(pw: PackedWeight, x: torch.Tensor, out: torch.Tensor, row_off: 
     _count()
 
 
+def _stream_args(sc: Scratch | None):
+    return (sc.partials, sc.tickets, sc.status) if sc is not None else (None, None, None)
+
+
 def moe_gate_up(pw: PackedWeight, h, norm_w, eps, act, items, n_items, top_k, z_max, scratch: Scratch | None = None) -> None:
     """Grouped expert gate|up GEMV with fused RMSNorm prologue and SwiGLU epilogue: act[pair] for every local pair."""
     accum, tickets = _accum_args(pw, 4 * z_max, scratch)
     if tickets is not None and z_max * pw.n_tiles > tickets.numel():
         accum, tickets = None, None
     stride = pw.n_tiles * pw.k_blocks * pw.chunk_bytes
-    ext().moe_gemv(pw.data, pw.fmt, pw.n, pw.k, stride, h, norm_w, eps, act, EPI_SWIGLU, items, n_items, top_k, z_max,
-                   accum, tickets, None, None, top_k, 0, 0, None, None, None)
-    _count()
+    _count(ext().moe_gemv(pw.data, pw.fmt, pw.n, pw.k, stride, h, norm_w, eps, act, EPI_SWIGLU, items, n_items, top_k, z_max,
+                          accum, tickets, None, None, top_k, 0, 0, None, None, None, *_stream_args(scratch)))
 
 
 def moe_down_combine(pw: PackedWeight, act, yslot, items, n_items, z_max, ids, wts, top_k, e0, n_local, h, tile_tickets,
                      scratch: Scratch | None = None, tp=None) -> None:
-    """Grouped expert down GEMV; the last CTA of each column tile combines the weighted pairs, all-reduces the tile
-    across expert-parallel ranks over peer memory (when ``tp`` is given) and adds it to the residual stream."""
+    """Grouped expert down GEMV and the weighted sum of the pairs into the residual stream.  With ``tp`` the last CTA of each column
+    tile does the sum and all-reduces the tile across expert-parallel ranks over peer memory."""
     accum, tickets = _accum_args(pw, 4 * z_max, scratch)
     if tickets is not None and z_max * pw.n_tiles > tickets.numel():
         accum, tickets = None, None
     stride = pw.n_tiles * pw.k_blocks * pw.chunk_bytes
-    ext().moe_gemv(pw.data, pw.fmt, pw.n, pw.k, stride, act, None, 0.0, yslot, EPI_MOE_COMBINE, items, n_items, 1, z_max,
-                   accum, tickets, ids, wts, top_k, e0, n_local, h, tile_tickets, tp)
-    _count()
+    _count(ext().moe_gemv(pw.data, pw.fmt, pw.n, pw.k, stride, act, None, 0.0, yslot, EPI_MOE_COMBINE, items, n_items, 1, z_max,
+                          accum, tickets, ids, wts, top_k, e0, n_local, h, tile_tickets, tp, *_stream_args(scratch)))
 
 
 def gemm(pw: PackedWeight, x: torch.Tensor, out: torch.Tensor, *, epi: int = EPI_STORE, bias: torch.Tensor | None = None,

@@ -19,7 +19,7 @@ BUILD_DIR = Path(__file__).resolve().parent / "_build"
 # mixers with a recurrent state, and experts
 DENSE, LATENT, GROUPED, MIXERS, EXPERTS = (f"llaminar_b200_{n}" for n in ("dense", "latent", "grouped", "mixers", "experts"))
 SOURCES = {
-    NAME: ["binding.cpp", "gemv.cu", "gemv_stream.cu", "gemm_tc.cu", "gemm_tc_small.cu", "gemm_tc_pair.cu", "attention.cu", "attention_tc.cu", "ops.cu", "gdn.cu", "moe_ep.cu", "no_alloc.cu"],
+    NAME: ["binding.cpp", "gemv.cu", "gemv_stream.cu", "gemm_tc.cu", "gemm_tc_small.cu", "gemm_tc_pair.cu", "attention.cu", "attention_tc.cu", "ops.cu", "gdn.cu", "moe_ep.cu", "moe_stream.cu", "no_alloc.cu"],
     DENSE: ["dense_binding.cpp", "dense_ops.cu"],
     LATENT: ["latent_binding.cpp", "latent_attention.cu", "latent_tc.cu"],
     GROUPED: ["grouped_binding.cpp", "grouped.cu", "attention.cu", "attention_tc.cu"],

@@ -157,10 +157,12 @@ static void gemm_tc_grouped(const Tensor& w, int64_t fmt, int64_t n, int64_t k, 
 }
 
 // Grouped expert GEMV over the router's work list: epi = EPI_SWIGLU (gate|up) or EPI_MOE_COMBINE (down + combine [+ all-reduce]).
-static void moe_gemv(const Tensor& w, int64_t fmt, int64_t n, int64_t k, int64_t expert_stride, const Tensor& x, const OptTensor& norm_w,
+// With `partials` calls without a tensor-parallel descriptor run the streaming kernel.  Returns the number of launches.
+static int64_t moe_gemv(const Tensor& w, int64_t fmt, int64_t n, int64_t k, int64_t expert_stride, const Tensor& x, const OptTensor& norm_w,
                      double eps, Tensor out, int64_t epi, const Tensor& items, const Tensor& n_items, int64_t x_div, int64_t z_max,
                      const OptTensor& accum, const OptTensor& tickets, const OptTensor& ids, const OptTensor& wts, int64_t top_k,
-                     int64_t e0, int64_t n_local, const OptTensor& h, const OptTensor& tile_tickets, const OptTensor& tp) {
+                     int64_t e0, int64_t n_local, const OptTensor& h, const OptTensor& tile_tickets, const OptTensor& tp, const OptTensor& partials,
+                     const OptTensor& unit_tickets, const OptTensor& status) {
     check_cuda(w, "w"); check_cuda(x, "x"); check_cuda(out, "out");
     const c10::cuda::CUDAGuard guard(x.device());
     TORCH_CHECK(k % 256 == 0, "k must be a multiple of 256");
@@ -200,7 +202,16 @@ static void moe_gemv(const Tensor& w, int64_t fmt, int64_t n, int64_t k, int64_t
     } else {
         TORCH_CHECK(epi == llm::EPI_SWIGLU && !p.out_f32, "grouped gate|up writes bf16 through the SwiGLU epilogue");
     }
+    if (partials.has_value() && unit_tickets.has_value()) {
+        const cudaError_t e = llm::launch_moe_stream(p, (int)z_max, mptr<float>(partials), (size_t)partials->numel(), mptr<unsigned>(unit_tickets),
+                                                     (size_t)unit_tickets->numel(), mptr<int>(status), cur_stream());
+        if (e != cudaErrorNotSupported) {
+            LLM_CUDA_CHECK(e);
+            return epi == llm::EPI_MOE_COMBINE ? 2 : 1;
+        }
+    }
     LLM_CUDA_CHECK(llm::launch_gemv(p, 4, (int)z_max, cur_stream()));
+    return 1;
 }
 
 static void dequant(const Tensor& w, int64_t fmt, int64_t n, int64_t k, Tensor out) {

@@ -7,7 +7,8 @@
 // shared-memory slots (it starts while the rows are quantised), rows are quantised once per item and CTA, and a tile split between CTAs is
 // finished by the one that holds its first chunk, which adds the others' parked sums in CTA order.  The weighted sum of the experts is
 // a launch of its own: inside this one it was a serial tail of the last CTA of every tile.
-// @TABLE@
+// Measured (128 experts of 768 x 2048, Q4_K, 8 tokens x 8 experts, one of eight layers in turn): gate | up 34.7 us (55.2 on the register
+// path), down and sum 26.2 us (35.6); what bounds it now is the dp4a arithmetic of four rows per chunk and the rows' quantisation.
 #include <cuda.h>
 
 #include "formats.cuh"
