@@ -180,6 +180,13 @@ class QLinear:
         """x: bf16 rows, or the fp32 residual rows when ``norm_w`` is given (GEMV path only).
         ``xn``: pre-normalised bf16 rows for the GEMM path."""
         rows = x.shape[0]
+        if len(self.parts) == 2 and epi == ops.EPI_STORE and scratch is not None and all(isinstance(w, PackedWeight) for w, _ in self.parts):
+            (a, _), (b, col) = self.parts
+            gemv = rows <= ops.GEMV_MAX_ROWS and xn is None
+            if gemv == (norm_w is not None) and ops.linear_dual(a, b, x if gemv or xn is None else xn, out[:, :col], out[:, col:col + b.n], scratch,
+                                                                norm_w=norm_w, eps=eps, bias_a=self.bias[:col] if self.bias is not None else None,
+                                                                bias_b=self.bias[col:col + b.n] if self.bias is not None else None):
+                return
         for w, col in self.parts:
             n = w.n if isinstance(w, PackedWeight) else w.shape[0]
             if epi == ops.EPI_SWIGLU:

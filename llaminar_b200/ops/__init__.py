@@ -205,6 +205,21 @@ def gemm(pw: PackedWeight, x: torch.Tensor, out: torch.Tensor, *, epi: int = EPI
     _count()
 
 
+DUAL_MAX_ROWS = 128
+
+
+def linear_dual(a: PackedWeight, b: PackedWeight, x: torch.Tensor, out_a: torch.Tensor, out_b: torch.Tensor, scratch: Scratch, *,
+                norm_w: torch.Tensor | None = None, eps: float = 1e-6, bias_a: torch.Tensor | None = None, bias_b: torch.Tensor | None = None) -> bool:
+    """Two matrices of different block formats on the same rows in one launch: the streaming GEMV with ``norm_w`` (up to GEMV_MAX_ROWS
+    fp32 rows), the small-batch GEMM without (bf16 rows, up to DUAL_MAX_ROWS).  False, and nothing done, where it does not fit."""
+    if x.shape[0] > (DUAL_MAX_ROWS if norm_w is None else GEMV_MAX_ROWS) or a.k != b.k:
+        return False
+    done = ext().linear_dual(a.data, a.fmt, a.n, b.data, b.fmt, b.n, a.k, x, norm_w, eps, out_a, out_b, bias_a, bias_b, scratch.tickets, scratch.partials, scratch.status)
+    if done:
+        _count()
+    return done
+
+
 def gemm_allgather(pw: PackedWeight, m_total: int, out: torch.Tensor, desc: torch.Tensor, *, epi: int = EPI_STORE,
                    bias: torch.Tensor | None = None, status: torch.Tensor | None = None) -> None:
     """Column-parallel GEMM with the all-gather of its row-sharded input fused into the launch (see AgFuse in gemm_tc.h)."""

@@ -538,6 +538,52 @@ static void gemm_tc(const Tensor& w, int64_t fmt, int64_t n, int64_t k, const Te
     LLM_CUDA_CHECK(llm::launch_gemm_tc(p, cur_stream()));
 }
 
+// Two matrices of different formats on the same rows in one launch: x bf16 (norm_w absent, up to 128 rows), or the fp32 residual rows and
+// the norm's gain (up to 4 rows).  False: not a call that one launch takes, nothing has been done.
+static bool linear_dual(const Tensor& w0, int64_t fmt0, int64_t n0, const Tensor& w1, int64_t fmt1, int64_t n1, int64_t k, const Tensor& x, const OptTensor& norm_w,
+                        double eps, Tensor out0, Tensor out1, const OptTensor& bias0, const OptTensor& bias1, const Tensor& tickets, const Tensor& partials,
+                        const Tensor& status) {
+    check_cuda(w0, "w0"); check_cuda(w1, "w1"); check_cuda(x, "x"); check_cuda(out0, "out0"); check_cuda(out1, "out1");
+    const c10::cuda::CUDAGuard guard(x.device());
+    TORCH_CHECK(k % 256 == 0, "k must be a multiple of 256");
+    TORCH_CHECK(partials.scalar_type() == torch::kFloat32 && tickets.scalar_type() == torch::kInt32 && status.scalar_type() == torch::kInt32, "scratch types");
+    const int64_t rows = x.size(0), tiles = (n0 + 127) / 128 + (n1 + 127) / 128;
+    if (tickets.numel() < tiles) return false;
+    cudaError_t e;
+    if (norm_w.has_value()) {
+        TORCH_CHECK(x.scalar_type() == torch::kFloat32 && norm_w->scalar_type() == torch::kFloat32, "fused norm: fp32 rows and gain");
+        auto params = [&](const Tensor& w, int64_t fmt, int64_t n, Tensor& out, const OptTensor& bias) {
+            llm::GemvParams p{};
+            p.w = static_cast<const uint8_t*>(w.data_ptr());
+            p.fmt = (int)fmt; p.n = (int)n; p.k = (int)k; p.n_tiles = (int)((n + 127) / 128); p.k_blocks = (int)(k / 256);
+            p.x = x.data_ptr(); p.x_stride = (int)x.stride(0); p.z_per_x = 1;
+            p.norm_w = cptr<float>(norm_w); p.eps = (float)eps; p.epi = llm::EPI_STORE; p.bias = cptr<float>(bias);
+            p.out = out.data_ptr(); p.out_stride = (int)out.stride(0); p.out_f32 = out.scalar_type() == torch::kFloat32;
+            return p;
+        };
+        e = llm::launch_gemv_stream_dual(params(w0, fmt0, n0, out0, bias0), params(w1, fmt1, n1, out1, bias1), (int)rows, static_cast<float*>(partials.data_ptr()),
+                                         (size_t)partials.numel(), reinterpret_cast<unsigned*>(tickets.data_ptr()), (size_t)tickets.numel(),
+                                         static_cast<int*>(status.data_ptr()), cur_stream());
+    } else {
+        TORCH_CHECK(x.scalar_type() == torch::kBFloat16 && x.is_contiguous(), "input must be contiguous bf16");
+        const int64_t slot_rows = rows <= 32 ? 32 : (rows <= 64 ? 64 : 128);        // two slots of [rows][128] for every CTA
+        if (partials.numel() < 148 * 2 * 128 * slot_rows) return false;
+        auto params = [&](const Tensor& w, int64_t fmt, int64_t n, Tensor& out, const OptTensor& bias) {
+            llm::GemmTcParams p{};
+            p.w = static_cast<const uint8_t*>(w.data_ptr()); p.fmt = (int)fmt; p.n = (int)n; p.k = (int)k; p.m = (int)rows;
+            p.x = static_cast<const __nv_bfloat16*>(x.data_ptr());
+            p.out = out.data_ptr(); p.out_stride = (int)out.stride(0); p.out_f32 = out.scalar_type() == torch::kFloat32;
+            p.epi = llm::EPI_STORE; p.bias = cptr<float>(bias); p.status = static_cast<int*>(status.data_ptr());
+            p.tickets = reinterpret_cast<unsigned*>(tickets.data_ptr()); p.partials = static_cast<float*>(partials.data_ptr());
+            return p;
+        };
+        e = llm::launch_gemm_tc_small_dual(params(w0, fmt0, n0, out0, bias0), params(w1, fmt1, n1, out1, bias1), cur_stream());
+    }
+    if (e == cudaErrorNotSupported) return false;
+    LLM_CUDA_CHECK(e);
+    return true;
+}
+
 // Column-parallel GEMM whose activation rows are all-gathered from the ranks inside the launch (AgFuse in gemm_tc.h).
 // `desc` is a host int64 tensor: [src ptr x8, avail ptr x8, stage ptr, staged ptr, world, rank, rows_per_rank, copy_ctas, epoch, spin_limit].
 static void gemm_tc_allgather(const Tensor& w, int64_t fmt, int64_t n, int64_t k, int64_t m, Tensor out, int64_t epi, const OptTensor& bias,
@@ -631,6 +677,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("moe_combine_sorted", &moe_combine_sorted);
     m.def("gemm_tc_grouped", &gemm_tc_grouped);
     m.def("gemm_tc", &gemm_tc);
+    m.def("linear_dual", &linear_dual);
     m.def("gemm_tc_allgather", &gemm_tc_allgather);
     m.def("gemm_tc_rs", &gemm_tc_rs);
     m.def("rs_reduce_norm", &rs_reduce_norm);

@@ -81,6 +81,9 @@ struct GemmTcParams {
 cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st);
 // small-batch kernel (block_m 32, 64 or 128), implemented in gemm_tc_small.cu
 cudaError_t launch_gemm_tc_small(const GemmTcParams& p, int block_m, int ksplit, cudaStream_t st);
+// two matrices of a mix of formats on the same rows (up to 128) in one launch; the slots and counters of `a` serve both
+// (a: tiles of a, then of b).  cudaErrorNotSupported: other formats or options, the caller launches one after the other
+cudaError_t launch_gemm_tc_small_dual(const GemmTcParams& a, const GemmTcParams& b, cudaStream_t st);
 // persistent kernel of CTA pairs for many rows and for the grouped mode (gemm_tc_pair.cu); `tokens`: rows of a tile, a multiple of 32 up to 256
 cudaError_t launch_gemm_tc_pair(const GemmTcParams& p, int tokens, cudaStream_t st);
 int gemm_pair_tokens(int fmt, int m, int n, int k);

@@ -157,8 +157,9 @@ struct UnitIter {
     }
 };
 
+// The work of CTA `cta` of the `ctas` that share the matrix.
 template <int FMT, int BM>
-__global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmTcParams p) {
+LLM_DEVICE void gemm_small_body(const CUtensorMap& tmap_x, const GemmTcParams& p, const int cta, const int ctas) {
     using C = Cfg<FMT, BM>;
     constexpr int R = C::RAW_SLOTS;
     extern __shared__ uint8_t smem_raw[];
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
     volatile int* abort_flag = s_abort;
     // optional timeline trace of CTA (flags >> 8): p.debug[role * 1024 + slot] = low 32 bits of the ns timer
     auto stamp = [&](int role, int slot) {
-        if (LLM_TRACE && p.debug && (int)blockIdx.x == (p.flags >> 8) && slot < 1024) {
+        if (LLM_TRACE && p.debug && cta == (p.flags >> 8) && slot < 1024) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
             p.debug[role * 1024 + slot] = (int)(t & 0x7fffffff);
@@ -220,12 +221,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
         if (LLM_TRACE && p.debug) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            p.debug[4096 + 4 * blockIdx.x + slot] = (int)(t & 0x7fffffff);
+            p.debug[4096 + 4 * cta + slot] = (int)(t & 0x7fffffff);
         }
     };
     if (tid == 0) cta_stamp(0);
     UnitIter it;
-    it.init(k_blocks, n_tiles, gridDim.x, blockIdx.x, streamk);
+    it.init(k_blocks, n_tiles, ctas, cta, streamk);
     Unit u;
 
     // chunk counter cc -> half of the operand ring (stages set*4 .. set*4+3) and the phase of its barriers
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
             const bool use_slots = p.partials != nullptr;
             const int c_first = u.contributors > 1 ? it.cta_of(u.tile * k_blocks) : 0;
             const int c_last = u.contributors > 1 ? it.cta_of(u.tile * k_blocks + k_blocks - 1) : 0;
-            const bool finisher = u.contributors > 1 && use_slots && (int)blockIdx.x == c_first;
+            const bool finisher = u.contributors > 1 && use_slots && cta == c_first;
             if (finisher) {
                 const unsigned target = (unsigned)(N_DQ_WARPS * (u.contributors - 1));
                 int got = 1;
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
                 // of its range) and the last arriver adds the slots up in CTA order; 4096 fp32 atomics per unit were
                 // measured to cost several microseconds when all CTAs reach their unit boundary together.
                 if (use_slots && !finisher) {
-                    float* mine = p.partials + ((size_t)blockIdx.x * 2 + (ui_ > 0 ? 1 : 0)) * (128 * BM);
+                    float* mine = p.partials + ((size_t)cta * 2 + (ui_ > 0 ? 1 : 0)) * (128 * BM);
 #pragma unroll
                     for (int i = 0; i < CW; ++i) __stcg(&mine[(c0 + i) * 128 + row], v[i]);
                 } else if (!use_slots) {
@@ -393,7 +394,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
                             for (int i = 0; i < CW; ++i) sum[i] += parked[j][i];
                         }
                         for (int c = c_first + MAX_C; c <= c_last; ++c) {        // more contributors than that: one by one
-                            if (c == (int)blockIdx.x) {
+                            if (c == cta) {
 #pragma unroll
                                 for (int i = 0; i < CW; ++i) sum[i] += v[i];
                             } else {
@@ -582,7 +583,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
             const int c_first = u.contributors > 1 ? it.cta_of(u.tile * k_blocks) : 0;
             const int c_last = u.contributors > 1 ? it.cta_of(u.tile * k_blocks + k_blocks - 1) : 0;
             const int nc = c_last - c_first + 1;
-            const bool finisher = u.contributors > 1 && (int)blockIdx.x == c_first;
+            const bool finisher = u.contributors > 1 && cta == c_first;
             auto slot_of = [&](int c) {
                 const int c_pos = (int)(((unsigned)c * (unsigned)it.total) / (unsigned)it.G);
                 return p.partials + ((size_t)c * 2 + (c_pos / k_blocks == u.tile ? 0 : 1)) * (128 * BM) + row;
@@ -634,7 +635,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
                 if (u.contributors > 1 && !finisher) {
-                    float* mine = p.partials + ((size_t)blockIdx.x * 2 + (ui_ > 0 ? 1 : 0)) * (128 * BM) + row;
+                    float* mine = p.partials + ((size_t)cta * 2 + (ui_ > 0 ? 1 : 0)) * (128 * BM) + row;
 #pragma unroll
                     for (int i = 0; i < 8; ++i) __stcg(mine + (m0 + i) * 128, v[i]);
                     continue;
@@ -818,7 +819,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
             // release (cumulative over the mbarrier) publishes them to that CTA
             int n = 0;
             while (it.next(u)) {
-                if (u.contributors > 1 && (int)blockIdx.x != it.cta_of(u.tile * k_blocks)) {
+                if (u.contributors > 1 && cta != it.cta_of(u.tile * k_blocks)) {
                     if (!mbar_wait(sig_bar, n & 1, abort_flag)) break;
                     red_release_gpu_add(&p.tickets[u.tile], (unsigned)N_DQ_WARPS);
                     ++n;
@@ -896,6 +897,21 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_
     if (tid == 0) cta_stamp(1);
 }
 
+template <int FMT, int BM>
+__global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ GemmTcParams p) {
+    gemm_small_body<FMT, BM>(tmap_x, p, blockIdx.x, gridDim.x);
+}
+
+// Two matrices of different formats on the same rows (the query / key and the value matrix of a 4-bit mix): the first `first` CTAs take one,
+// the others the other.  Apart from its bytes a launch of this kernel costs some 10 us (fill, split tiles, drain), and the second matrix
+// is a small one.  5120 and 1024 x 4096, Q4_K and Q6_K in every second layer, 32 rows: 13.3 us a layer on average, 20.8 with a launch each.
+template <int FA, int FB, int BM>
+__global__ void __launch_bounds__(THREADS, 1) gemm_tc_small_dual_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ GemmTcParams a,
+                                                                        const __grid_constant__ GemmTcParams b, const int first) {
+    if ((int)blockIdx.x < first) gemm_small_body<FA, BM>(tmap_x, a, blockIdx.x, first);
+    else gemm_small_body<FB, BM>(tmap_x, b, blockIdx.x - first, gridDim.x - first);
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -911,22 +927,26 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-template <int FMT, int BM>
-static cudaError_t launch_one(const GemmTcParams& p, int ksplit, cudaStream_t st) {
-    using C = Cfg<FMT, BM>;
+template <int BM>
+static bool rows_map(CUtensorMap* tmap, const GemmTcParams& p) {
     EncodeTiledFn enc = encode_fn();
-    if (!enc) return cudaErrorNotSupported;
-    static_assert(C::CHUNK % 16 == 0 && C::RING_BYTES % 16 == 0, "bulk copies need 16-byte granularity");
-    if (reinterpret_cast<uintptr_t>(p.w) & 15) return cudaErrorInvalidValue;      // the chunks arrive by bulk copy
-    CUtensorMap tmap;
     const cuuint64_t dims[2] = {(cuuint64_t)p.k, (cuuint64_t)p.m};
     const cuuint64_t strides[1] = {(cuuint64_t)p.k * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)BM};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(&tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p.x), dims, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    return enc && enc(tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p.x), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int FMT, int BM>
+static cudaError_t launch_one(const GemmTcParams& p, int ksplit, cudaStream_t st) {
+    using C = Cfg<FMT, BM>;
+    if (!encode_fn()) return cudaErrorNotSupported;
+    static_assert(C::CHUNK % 16 == 0 && C::RING_BYTES % 16 == 0, "bulk copies need 16-byte granularity");
+    if (reinterpret_cast<uintptr_t>(p.w) & 15) return cudaErrorInvalidValue;      // the chunks arrive by bulk copy
+    CUtensorMap tmap;
+    if (!rows_map<BM>(&tmap, p)) return cudaErrorInvalidValue;
     static bool attr_set = false;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(gemm_tc_small_kernel<FMT, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
@@ -969,7 +989,51 @@ static cudaError_t launch_fmt(const GemmTcParams& p, int bm, int ks, cudaStream_
     return cudaErrorInvalidValue;
 }
 
+template <int FA, int FB, int BM>
+static cudaError_t launch_dual(const GemmTcParams& a, const GemmTcParams& b, cudaStream_t st) {
+    CUtensorMap tmap;
+    if (!rows_map<BM>(&tmap, a)) return cudaErrorNotSupported;
+    constexpr int SMEM = Cfg<FA, BM>::SMEM_BYTES > Cfg<FB, BM>::SMEM_BYTES ? Cfg<FA, BM>::SMEM_BYTES : Cfg<FB, BM>::SMEM_BYTES;
+    static bool attr_set = false;
+    if (!attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_tc_small_dual_kernel<FA, FB, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e != cudaSuccess) return e;
+        attr_set = true;
+    }
+    // CTAs by bytes, at least four chunks per CTA and at most four CTAs per tile, as for one matrix
+    const int kb = a.k / 256, ta = (a.n + 127) / 128, tb = (b.n + 127) / 128;
+    auto most = [&](int tiles) { const int g1 = (tiles * kb + 3) / 4, g2 = 4 * tiles; return g1 < g2 ? g1 : g2; };
+    const double wa = (double)ta * Cfg<FA, BM>::CHUNK, wb = (double)tb * Cfg<FB, BM>::CHUNK;
+    int gb = (int)(148 * wb / (wa + wb) + 0.5);
+    if (gb > most(tb)) gb = most(tb);
+    if (gb < 1) gb = 1;
+    int ga = 148 - gb;
+    if (ga > most(ta)) ga = most(ta);
+    if (ga < 1 || gb > 147) return cudaErrorNotSupported;
+    if ((unsigned long long)((long long)(ta > tb ? ta : tb) * kb + 1) * 148ull >= (1ull << 32)) return cudaErrorNotSupported;       // 32-bit work indices
+    GemmTcParams qa = a, qb = b;
+    qa.flags = qb.flags = 2;                         // split tiles
+    qb.partials = a.partials + (size_t)ga * 2 * 128 * BM;
+    qb.tickets = a.tickets + ta;
+    return launch_pdl(gemm_tc_small_dual_kernel<FA, FB, BM>, dim3(ga + gb), dim3(THREADS), SMEM, st, tmap, qa, qb, ga);
+}
+
+template <int FA, int FB>
+static cudaError_t launch_dual_rows(const GemmTcParams& a, const GemmTcParams& b, cudaStream_t st) {
+    return a.m <= 32 ? launch_dual<FA, FB, 32>(a, b, st) : a.m <= 64 ? launch_dual<FA, FB, 64>(a, b, st) : launch_dual<FA, FB, 128>(a, b, st);
+}
+
 }  // namespace tcs
+
+cudaError_t launch_gemm_tc_small_dual(const GemmTcParams& a, const GemmTcParams& b, cudaStream_t st) {
+    if (a.m < 1 || a.m > 128 || a.m != b.m || a.k != b.k || a.x != b.x || a.epi != EPI_STORE || b.epi != EPI_STORE || a.tp || b.tp || !a.partials || !a.tickets ||
+        ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(b.w) | reinterpret_cast<uintptr_t>(a.x)) & 15))
+        return cudaErrorNotSupported;
+    if (a.fmt == FMT_Q4_K && b.fmt == FMT_Q6_K) return tcs::launch_dual_rows<FMT_Q4_K, FMT_Q6_K>(a, b, st);
+    if (a.fmt == FMT_Q4_K && b.fmt == FMT_Q5_K) return tcs::launch_dual_rows<FMT_Q4_K, FMT_Q5_K>(a, b, st);
+    if (a.fmt == FMT_Q5_K && b.fmt == FMT_Q6_K) return tcs::launch_dual_rows<FMT_Q5_K, FMT_Q6_K>(a, b, st);
+    return cudaErrorNotSupported;
+}
 
 cudaError_t launch_gemm_tc_small(const GemmTcParams& p, int bm, int ks, cudaStream_t st) {
     switch (p.fmt) {

@@ -63,6 +63,10 @@ cudaError_t launch_gemv(const GemvParams& p, int m_tile, int z, cudaStream_t st)
 // Streaming kernel for plain dense calls (gemv_stream.cu): one persistent CTA per SM, chunks by bulk copy.  Returns
 // cudaErrorNotSupported for calls it does not take (grouped experts, fused tensor-parallel epilogue, missing scratch).
 cudaError_t launch_gemv_stream(const GemvParams& p, int m, float* partials, size_t partials_floats, unsigned* tickets, int* status, cudaStream_t st);
+// Two matrices of a mix of formats on the same normalised rows in one launch (gemv_stream.cu); counters: tiles of a, then of b.
+// cudaErrorNotSupported as above: the caller launches one after the other.
+cudaError_t launch_gemv_stream_dual(const GemvParams& a, const GemvParams& b, int m, float* partials, size_t partials_floats, unsigned* tickets, size_t n_tickets,
+                                    int* status, cudaStream_t st);
 // Streaming kernel for the routed experts of a decode step (moe_stream.cu): gate | up with SwiGLU, or down and the weighted sum (two
 // launches); z_max: capacity of the work list.  cudaErrorNotSupported as above.
 cudaError_t launch_moe_stream(const GemvParams& p, int z_max, float* partials, size_t partials_floats, unsigned* tickets, size_t n_tickets, int* status, cudaStream_t st);

@@ -162,8 +162,9 @@ LLM_DEVICE void quantise_acts(const GemvParams& p, int kb_first, int n_act, int 
     bar_compute();
 }
 
+// The work of CTA `cta` of the `ctas` that share the matrix.
 template <int FMT, int M, int NORM>
-__global__ void __launch_bounds__(THREADS, 1) gemv_stream_kernel(const GemvParams p, const Extra e) {
+LLM_DEVICE void gemv_stream_body(const GemvParams& p, const Extra& e, const int cta_, const int ctas) {
     constexpr int CHUNK = FmtTraits<FMT>::CHUNK;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t s_full[8], s_empty[8];
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_stream_kernel(const GemvParam
     __syncthreads();
     volatile int* abort_flag = s_abort;
     Walk it;
-    it.init(p.k_blocks, p.n_tiles, gridDim.x, blockIdx.x);
+    it.init(p.k_blocks, p.n_tiles, ctas, cta_);
     Unit u;
 
     if (warp == N_WARPS) {
@@ -254,9 +255,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_stream_kernel(const GemvParam
             for (int m = 0; m < M; ++m) v[m] = red[m * 128 + tid] + red[(M + m) * 128 + tid] + red[(2 * M + m) * 128 + tid] + red[(3 * M + m) * 128 + tid];
             const int row = u.tile * 128 + tid;
             if (u.first_cta != u.last_cta) {
-                if ((int)blockIdx.x != u.first_cta) {
+                if (cta_ != u.first_cta) {
                     // park and tell the finisher (every thread's stores, then one release from thread 0)
-                    float* mine = e.partials + (size_t)blockIdx.x * (4 * 128);
+                    float* mine = e.partials + (size_t)cta_ * (4 * 128);
 #pragma unroll
                     for (int m = 0; m < M; ++m) __stcg(&mine[m * 128 + tid], v[m]);
                     __threadfence();
@@ -317,6 +318,21 @@ __global__ void __launch_bounds__(THREADS, 1) gemv_stream_kernel(const GemvParam
     }
 }
 
+template <int FMT, int M, int NORM>
+__global__ void __launch_bounds__(THREADS, 1) gemv_stream_kernel(const __grid_constant__ GemvParams p, const __grid_constant__ Extra e) {
+    gemv_stream_body<FMT, M, NORM>(p, e, blockIdx.x, gridDim.x);
+}
+
+// Two matrices of different formats on the same normalised rows (the query / key and the value matrix of a 4-bit mix): the first `first`
+// CTAs take one, the others the other.  5120 and 1024 x 4096, Q4_K and Q6_K in every second layer, one row: 7.1 us a layer on average,
+// 12.9 with a launch each.
+template <int FA, int FB, int M>
+__global__ void __launch_bounds__(THREADS, 1) gemv_stream_dual_kernel(const __grid_constant__ GemvParams a, const __grid_constant__ Extra ea,
+                                                                      const __grid_constant__ GemvParams b, const __grid_constant__ Extra eb, const int first) {
+    if ((int)blockIdx.x < first) gemv_stream_body<FA, M, 1>(a, ea, blockIdx.x, first);
+    else gemv_stream_body<FB, M, 1>(b, eb, blockIdx.x - first, gridDim.x - first);
+}
+
 static size_t smem_bytes(int chunk, int slots, int m, int act_cap) {
     return (size_t)slots * chunk + (size_t)m * act_cap * sizeof(ActBlk) + 2 * 4 * (size_t)m * 128 * sizeof(float) + 512 * sizeof(uint32_t);
 }
@@ -335,16 +351,23 @@ template <int FMT, int M>
 static cudaError_t launch_m(const GemvParams& p, const Extra& e, int grid, size_t smem, cudaStream_t st) {
     return p.norm_w ? launch_k<FMT, M, 1>(p, e, grid, smem, st) : launch_k<FMT, M, 0>(p, e, grid, smem, st);
 }
+// Ring and activation blocks of a CTA with that many chunks; slots = 0: they do not fit
+template <int FMT>
+static Extra ring(const GemvParams& p, int m, int chunks_per_cta, float* partials, unsigned* tickets, int* status, size_t* smem) {
+    constexpr int CHUNK = FmtTraits<FMT>::CHUNK;
+    Extra e{partials, tickets, status, 8, 0};
+    e.act_cap = p.k_blocks < chunks_per_cta ? p.k_blocks : chunks_per_cta;
+    *smem = smem_bytes(CHUNK, 8, m, e.act_cap);
+    if (*smem > 216 * 1024) { e.slots = 4; *smem = smem_bytes(CHUNK, 4, m, e.act_cap); }
+    if (*smem > 216 * 1024) e.slots = 0;
+    return e;
+}
 template <int FMT>
 static cudaError_t launch_f(const GemvParams& p, int m, int grid, int chunks_per_cta, float* partials, unsigned* tickets, int* status,
                             cudaStream_t st) {
-    constexpr int CHUNK = FmtTraits<FMT>::CHUNK;
-    Extra e{partials, tickets, status, 0, 0};
-    e.act_cap = p.k_blocks < chunks_per_cta ? p.k_blocks : chunks_per_cta;
-    e.slots = 8;
-    size_t smem = smem_bytes(CHUNK, 8, m, e.act_cap);
-    if (smem > 216 * 1024) { e.slots = 4; smem = smem_bytes(CHUNK, 4, m, e.act_cap); }
-    if (smem > 216 * 1024) return cudaErrorNotSupported;
+    size_t smem = 0;
+    const Extra e = ring<FMT>(p, m, chunks_per_cta, partials, tickets, status, &smem);
+    if (!e.slots) return cudaErrorNotSupported;
     switch (m) {
         case 1: return launch_m<FMT, 1>(p, e, grid, smem, st);
         case 2: return launch_m<FMT, 2>(p, e, grid, smem, st);
@@ -354,7 +377,55 @@ static cudaError_t launch_f(const GemvParams& p, int m, int grid, int chunks_per
     return cudaErrorInvalidValue;
 }
 
+template <int FA, int FB, int M>
+static cudaError_t launch_dual_m(const GemvParams& a, const Extra& ea, const GemvParams& b, const Extra& eb, int ga, int gb, size_t smem, cudaStream_t st) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        const cudaError_t err = cudaFuncSetAttribute(gemv_stream_dual_kernel<FA, FB, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        if (err != cudaSuccess) return err;
+        attr_set = true;
+    }
+    return launch_pdl(gemv_stream_dual_kernel<FA, FB, M>, dim3(ga + gb), dim3(THREADS), smem, st, a, ea, b, eb, ga);
+}
+template <int FA, int FB>
+static cudaError_t launch_dual(const GemvParams& a, const GemvParams& b, int m, float* partials, unsigned* tickets, int* status, cudaStream_t st) {
+    // CTAs by bytes, at least four chunks per CTA, as for one matrix
+    const int ca = a.n_tiles * a.k_blocks, cb = b.n_tiles * b.k_blocks;
+    const double wa = (double)ca * FmtTraits<FA>::CHUNK, wb = (double)cb * FmtTraits<FB>::CHUNK;
+    int gb = (int)(148 * wb / (wa + wb) + 0.5);
+    if (gb > cb / 4) gb = cb / 4;
+    if (gb < 1) gb = 1;
+    int ga = 148 - gb;
+    if (ga > ca / 4) ga = ca / 4;
+    if (ga < 1) ga = 1;
+    size_t sa = 0, sb = 0;
+    const Extra ea = ring<FA>(a, m, (ca + ga - 1) / ga + 1, partials, tickets, status, &sa);
+    const Extra eb = ring<FB>(b, m, (cb + gb - 1) / gb + 1, partials + (size_t)ga * 4 * 128, tickets + a.n_tiles, status, &sb);
+    if (!ea.slots || !eb.slots) return cudaErrorNotSupported;
+    const size_t smem = sa > sb ? sa : sb;
+    switch (m) {
+        case 1: return launch_dual_m<FA, FB, 1>(a, ea, b, eb, ga, gb, smem, st);
+        case 2: return launch_dual_m<FA, FB, 2>(a, ea, b, eb, ga, gb, smem, st);
+        case 3: return launch_dual_m<FA, FB, 3>(a, ea, b, eb, ga, gb, smem, st);
+        case 4: return launch_dual_m<FA, FB, 4>(a, ea, b, eb, ga, gb, smem, st);
+    }
+    return cudaErrorNotSupported;
+}
+
 }  // namespace gs
+
+cudaError_t launch_gemv_stream_dual(const GemvParams& a, const GemvParams& b, int m, float* partials, size_t partials_floats, unsigned* tickets, size_t n_tickets,
+                                    int* status, cudaStream_t st) {
+    if (!partials || !tickets || !a.norm_w || a.norm_w != b.norm_w || a.x != b.x || a.k != b.k || a.tp || b.tp || a.items || b.items || a.expert_ids || b.expert_ids ||
+        a.epi != EPI_STORE || b.epi != EPI_STORE || ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(b.w)) & 15) ||
+        (size_t)148 * 4 * 128 > partials_floats || (size_t)(a.n_tiles + b.n_tiles) > n_tickets ||
+        (unsigned long long)((long long)(a.n_tiles > b.n_tiles ? a.n_tiles : b.n_tiles) * a.k_blocks + 1) * 148ull >= (1ull << 32))
+        return cudaErrorNotSupported;
+    if (a.fmt == FMT_Q4_K && b.fmt == FMT_Q6_K) return gs::launch_dual<FMT_Q4_K, FMT_Q6_K>(a, b, m, partials, tickets, status, st);
+    if (a.fmt == FMT_Q4_K && b.fmt == FMT_Q5_K) return gs::launch_dual<FMT_Q4_K, FMT_Q5_K>(a, b, m, partials, tickets, status, st);
+    if (a.fmt == FMT_Q5_K && b.fmt == FMT_Q6_K) return gs::launch_dual<FMT_Q5_K, FMT_Q6_K>(a, b, m, partials, tickets, status, st);
+    return cudaErrorNotSupported;
+}
 
 // cudaErrorNotSupported: the call is not one this kernel takes (the caller falls back to launch_gemv).
 cudaError_t launch_gemv_stream(const GemvParams& p, int m, float* partials, size_t partials_floats, unsigned* tickets, int* status, cudaStream_t st) {
