@@ -546,7 +546,7 @@ class CudaModel:
         else:
             kv_bf16, btab = self._kv_for_prefill(fb, kv_layer)
             ops.attn_prefill(q, kv_bf16, o3, btab, fb.cu_q, fb.ctx_lens, self.n_heads_local,
-                             self.n_kv_local, c.head_dim, scale, fb.max_q_len, scratch=self.scratch)
+                             self.n_kv_local, c.head_dim, scale, fb.max_q_len, scratch=self.scratch, max_kv_len=fb.max_kv_len)
         return o
 
     def _linear_attention(self, L: CudaLayer, fb: ForwardBatch, inp: torch.Tensor, T: int) -> torch.Tensor:
@@ -622,7 +622,7 @@ class CudaModel:
             if fb.is_decode:
                 ops.attn_decode(qb, kv_layer, o3, fb.block_table, fb.seq_lens, H, Hk, D, fb.rows_per_seq, scale, fb.n_splits, self.scratch)
             else:
-                ops.attn_prefill(qb, kv_layer, o3, fb.block_table, fb.cu_q, fb.ctx_lens, H, Hk, D, scale, fb.max_q_len, scratch=self.scratch)
+                ops.attn_prefill(qb, kv_layer, o3, fb.block_table, fb.cu_q, fb.ctx_lens, H, Hk, D, scale, fb.max_q_len, scratch=self.scratch, max_kv_len=fb.max_kv_len)
         if gate is not None:
             o.copy_(o.float() * torch.sigmoid(gate))
         return o

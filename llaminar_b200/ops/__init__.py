@@ -278,15 +278,17 @@ def attn_decode(q, kv, out, block_table, seq_lens, n_heads, n_kv_heads, head_dim
 
 
 def attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, head_dim, scale, max_q_len,
-                 tensor_core: bool | None = None, scratch: "Scratch | None" = None) -> None:
+                 tensor_core: bool | None = None, scratch: "Scratch | None" = None, max_kv_len: int = 0) -> None:
     """Causal GQA attention of a prefill chunk over the paged cache.  ``tensor_core`` picks the tcgen05 kernel (head_dim 128),
     otherwise the mma.sync kernel runs.  Default: the tcgen05 kernel wherever it fits; it is the faster one from ATTN_TC_MIN_ROWS
     query rows on (32 / 8 heads: 8.9 vs 11.3 us at 16 rows, 23.6 vs 82.6 at 1024, 164 vs 785 at 4096, 120 vs 414 at 500 rows
-    behind 7000 tokens); LLAMINAR_ATTN_TC=0 turns it off."""
+    behind 7000 tokens); LLAMINAR_ATTN_TC=0 turns it off.  With ``max_kv_len`` (the longest context and chunk of the batch; 0:
+    unknown) and ``scratch`` it shares the keys of few query rows out between CTAs."""
     if tensor_core is None:
         tensor_core = head_dim == 128 and max_q_len >= ATTN_TC_MIN_ROWS and _attn_tc_default()
     status = scratch.status if (tensor_core and scratch is not None) else None
-    ext().attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, head_dim, scale, max_q_len, bool(tensor_core), status)
+    ext().attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, head_dim, scale, max_q_len, bool(tensor_core), status,
+                       max_kv_len, scratch.part_o if status is not None else None, scratch.part_ml if status is not None else None)
     _count()
 
 

@@ -60,7 +60,8 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
     __shared__ int s_abort[2];       // [1] stays 0 here (tc_common.cuh: restarts the wait clock when set)
     pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int kvh = blockIdx.y, seq = blockIdx.z, G = p.n_heads / p.n_kv_heads;
+    const int splits = max(1, p.splits), seq = blockIdx.z / splits, split = blockIdx.z - seq * splits;
+    const int kvh = blockIdx.y, G = p.n_heads / p.n_kv_heads;
     const int q_start = p.cu_q[seq], q_len = p.cu_q[seq + 1] - q_start;
     // slot z of this sequence and K/V head: query tile z / G, head z % G of the group.  The last query tiles see the most keys: they
     // go first so that the grid ends with the short CTAs.
@@ -71,8 +72,16 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
     const int ctx = p.ctx_lens[seq];                       // tokens already in the cache before this chunk
     const int q_lo = first / G * BQ, q_hi = min(((both ? first + 1 : first) / G + 1) * BQ, q_len);
     const int kv_end = ctx + q_hi;                         // keys the CTA's rows can see
-    const int tile0 = first_key(ctx + q_lo, p.window, p.chunk) / BK;          // tile of the first key that its first row sees
-    const int nt = (kv_end + BK - 1) / BK - tile0, n_pages = (kv_end + PAGE - 1) / PAGE;
+    const int tile_lo = first_key(ctx + q_lo, p.window, p.chunk) / BK;        // tile of the first key that its first row sees
+    const int tile_hi = (kv_end + BK - 1) / BK, n_pages = (kv_end + PAGE - 1) / PAGE;
+    const int per = (tile_hi - tile_lo + splits - 1) / splits, tile0 = tile_lo + split * per, nt = min(tile_hi, tile0 + per) - tile0;
+    // where this CTA's first slot parks its results, if the keys are shared out
+    const size_t part = (((size_t)(seq * p.n_kv_heads + kvh) * gridDim.x + first / 2) * 2 * splits + split) * BQ;
+    if (nt <= 0) {                                         // fewer tiles than splits
+        for (int i = threadIdx.x; i < 2 * BQ; i += THREADS)
+            *reinterpret_cast<float2*>(p.part_ml + (part + (size_t)(i / BQ) * splits * BQ + i % BQ) * 2) = make_float2(-INFINITY, 0.f);
+        return;
+    }
     const int* btab = p.block_table + (size_t)seq * p.max_pages;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bars = smem_u32(s_bars);
@@ -191,7 +200,20 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
                 mbar_arrive_if(bar(P_FULL + slot), lane == 0);
             }
             ok = ok && mbar_wait_warp(bar(O_FULL + slot), 0, abort_flag);
-            if (ok) {
+            if (ok && splits > 1) {
+                tc_fence_after();
+                const size_t at = part + (size_t)slot * splits * BQ + row;
+                float4* dst = reinterpret_cast<float4*>(p.part_o + at * D);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t r[32];
+                    tmem_ld_n<32>(t_o + c * 32, r);
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        dst[c * 8 + u] = make_float4(__uint_as_float(r[4 * u]), __uint_as_float(r[4 * u + 1]), __uint_as_float(r[4 * u + 2]), __uint_as_float(r[4 * u + 3]));
+                }
+                *reinterpret_cast<float2*>(p.part_ml + at * 2) = make_float2(m, l);
+            } else if (ok) {
                 tc_fence_after();
                 if (p.sink) l += exp2f(p.sink[head] * LOG2E - m);
                 float inv = l > 0.f ? 1.f / l : 0.f;
@@ -298,7 +320,58 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
     if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
+// The splits' results of a query row, a warp per row and head: rescaled to the largest maximum, summed up in split order.
+__global__ void __launch_bounds__(128) paged_attn_prefill_merge_kernel(const AttnPrefillParams p, int pairs) {
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, G = p.n_heads / p.n_kv_heads, head = blockIdx.y, kvh = head / G, seq = blockIdx.z;
+    const int q_start = p.cu_q[seq], q_len = p.cu_q[seq + 1] - q_start;
+    const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (r >= q_len) return;
+    const int z = r / BQ * G + head % G;                    // the row's slot
+    const size_t part = (((size_t)(seq * p.n_kv_heads + kvh) * pairs * 2 + z) * p.splits) * BQ + r % BQ;
+    float m = -INFINITY;
+    for (int s = 0; s < p.splits; ++s) m = fmaxf(m, __ldcg(p.part_ml + (part + (size_t)s * BQ) * 2));
+    float l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int s = 0; s < p.splits; ++s) {
+        const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (part + (size_t)s * BQ) * 2));
+        const float c = ml.x == -INFINITY ? 0.f : exp2f(ml.x - m);
+        if (ml.x == -INFINITY && ml.y == 0.f) continue;     // no keys there
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.part_o + (part + (size_t)s * BQ) * D) + lane);
+        l += c * ml.y;
+        o[0] += c * v.x; o[1] += c * v.y; o[2] += c * v.z; o[3] += c * v.w;
+    }
+    const size_t at = (size_t)(q_start + r);
+    if (p.sink) l += exp2f(p.sink[head] * LOG2E - m);
+    float inv = l > 0.f ? 1.f / l : 0.f;
+    if (p.gate && p.gate_heads) inv *= __fdividef(1.f, 1.f + __expf(-__bfloat162float(p.gate[at * p.gate_row + head])));
+    if (p.gate && !p.gate_heads) {
+        const uint2 g = *reinterpret_cast<const uint2*>(p.gate + at * p.gate_row + head * D + lane * 4);
+        o[0] *= __fdividef(1.f, 1.f + __expf(-bf16_lo(g.x))); o[1] *= __fdividef(1.f, 1.f + __expf(-bf16_hi(g.x)));
+        o[2] *= __fdividef(1.f, 1.f + __expf(-bf16_lo(g.y))); o[3] *= __fdividef(1.f, 1.f + __expf(-bf16_hi(g.y)));
+    }
+    *reinterpret_cast<uint2*>(p.out + (at * p.n_heads + head) * D + lane * 4) = make_uint2(pack_bf16(o[0] * inv, o[1] * inv), pack_bf16(o[2] * inv, o[3] * inv));
+}
+
+static int pairs_of(int n_heads, int n_kv_heads, int max_q_len) { return ((max_q_len + BQ - 1) / BQ * (n_heads / n_kv_heads) + 1) / 2; }
+
 }  // namespace atc
+
+// A pair of query tiles walks its keys at 1.5 us per tile of 128 whatever else the GPU does: where the pairs leave SMs without a CTA, the
+// keys are shared out, at least four tiles to a split (500 rows behind 7000 tokens, 32 / 8 heads: 116 -> 76 us;
+// 16 rows behind 7000: 105 -> 28.5; 200 rows of two sequences behind 6000: 97 -> 65).
+int attn_prefill_tc_splits(int n_heads, int n_kv_heads, int n_seqs, int max_q_len, int max_kv_len, long long part_o, long long part_ml) {
+    if (n_kv_heads < 1 || n_heads % n_kv_heads || n_seqs < 1 || max_q_len < 1) return 1;
+    const long long ctas = (long long)atc::pairs_of(n_heads, n_kv_heads, max_q_len) * n_kv_heads * n_seqs, slots = 2 * ctas;
+    long long s = 148 / ctas;
+    const long long by_keys = max_kv_len / (4 * atc::BK), by_o = part_o / (slots * atc::BQ * atc::D), by_ml = part_ml / (slots * atc::BQ * 2);
+    if (s > by_keys) s = by_keys;
+    if (s > by_o) s = by_o;
+    if (s > by_ml) s = by_ml;
+    if (s > 16) s = 16;
+    return s < 2 ? 1 : (int)s;
+}
 
 cudaError_t launch_attn_prefill_tc(const AttnPrefillParams& p, int n_seqs, int max_q_len, int* status, cudaStream_t st) {
     if (n_seqs == 0 || max_q_len == 0) return cudaSuccess;
@@ -306,7 +379,9 @@ cudaError_t launch_attn_prefill_tc(const AttnPrefillParams& p, int n_seqs, int m
     // the cache as a matrix of head_dim columns: 64 rows per page, K or V, and head
     CUtensorMap map;
     if (!tc5::make_map(&map, p.kv, atc::D, (uint64_t)p.n_pages * 2 * p.n_kv_heads * atc::PAGE, atc::D, atc::PAGE)) return cudaErrorInvalidValue;
-    const dim3 grid(((max_q_len + atc::BQ - 1) / atc::BQ * (p.n_heads / p.n_kv_heads) + 1) / 2, p.n_kv_heads, n_seqs);
+    const int splits = p.splits > 1 ? p.splits : 1;
+    const dim3 grid(atc::pairs_of(p.n_heads, p.n_kv_heads, max_q_len), p.n_kv_heads, n_seqs * splits);
+    if (splits > 1 && (!p.part_o || !p.part_ml || ((reinterpret_cast<uintptr_t>(p.part_o) | reinterpret_cast<uintptr_t>(p.part_ml)) & 15))) return cudaErrorInvalidValue;
     auto go = [&](auto kernel, bool& once) -> cudaError_t {
         if (!once) {
             cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, atc::SMEM_BYTES);
@@ -316,7 +391,9 @@ cudaError_t launch_attn_prefill_tc(const AttnPrefillParams& p, int n_seqs, int m
         return launch_pdl(kernel, grid, dim3(atc::THREADS), atc::SMEM_BYTES, st, map, p, status);
     };
     static bool plain = false, capped = false;
-    return p.softcap > 0.f ? go(atc::paged_attn_prefill_tc_kernel<true>, capped) : go(atc::paged_attn_prefill_tc_kernel<false>, plain);
+    const cudaError_t e = p.softcap > 0.f ? go(atc::paged_attn_prefill_tc_kernel<true>, capped) : go(atc::paged_attn_prefill_tc_kernel<false>, plain);
+    if (e != cudaSuccess || splits == 1) return e;
+    return launch_pdl(atc::paged_attn_prefill_merge_kernel, dim3((max_q_len + 3) / 4, p.n_heads, n_seqs), dim3(128), 0, st, p, (int)grid.x);
 }
 
 LLM_DEFINE_BOUNDS_STATUS_READER(bounds_status_attention_tc)

@@ -371,7 +371,7 @@ static void attn_decode(const Tensor& q, const Tensor& kv, Tensor out, const Ten
 
 static void attn_prefill(const Tensor& q, const Tensor& kv, Tensor out, const Tensor& block_table, const Tensor& cu_q,
                          const Tensor& ctx_lens, int64_t n_heads, int64_t n_kv_heads, int64_t head_dim, double scale, int64_t max_q_len,
-                         bool tensor_core, const OptTensor& status) {
+                         bool tensor_core, const OptTensor& status, int64_t max_kv_len, const OptTensor& part_o, const OptTensor& part_ml) {
     check_cuda(q, "q");
     const c10::cuda::CUDAGuard guard(q.device());
     llm::AttnPrefillParams p{};
@@ -383,6 +383,11 @@ static void attn_prefill(const Tensor& q, const Tensor& kv, Tensor out, const Te
     p.scale = (float)scale; p.n_pages = (int)kv.size(0);
     if (tensor_core) {
         TORCH_CHECK(head_dim == 128, "the tcgen05 prefill attention is built for head_dim 128");
+        if (part_o.has_value() && part_ml.has_value() && max_kv_len > 0) {
+            TORCH_CHECK(part_o->scalar_type() == torch::kFloat32 && part_ml->scalar_type() == torch::kFloat32, "attention scratch must be fp32");
+            p.splits = llm::attn_prefill_tc_splits(p.n_heads, p.n_kv_heads, (int)ctx_lens.numel(), (int)max_q_len, (int)max_kv_len, part_o->numel(), part_ml->numel());
+            p.part_o = mptr<float>(part_o); p.part_ml = mptr<float>(part_ml);
+        }
         LLM_CUDA_CHECK(llm::launch_attn_prefill_tc(p, (int)ctx_lens.numel(), (int)max_q_len, mptr<int>(status), cur_stream()));
     } else {
         LLM_CUDA_CHECK(llm::launch_attn_prefill(p, (int)ctx_lens.numel(), (int)max_q_len, cur_stream()));

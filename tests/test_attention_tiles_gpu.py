@@ -70,6 +70,19 @@ def test_tiles(heads, kv_heads, lens, ctx, rising):
     _check(out, q, cu, c, keys, values)
 
 
+@pytest.mark.parametrize("heads,kv_heads,lens,ctx", [(8, 2, [1], [4000]), (7, 1, [130, 3], [1100, 2000]), (4, 4, [17, 250], [513, 0]), (32, 8, [40], [5000])])
+def test_keys_shared_out(heads, kv_heads, lens, ctx):
+    """Few query rows behind many keys: splits of equal tiles, a ragged last one, sequences with fewer tiles than splits."""
+    from llaminar_b200 import ops
+    q, kv, table, cu, c, keys, values = _case(heads, kv_heads, lens, ctx, True, 2)
+    sc, outs = ops.scratch_for(DEV), []
+    for longest in (0, max(n + m for n, m in zip(lens, ctx))):
+        outs.append(torch.full_like(q, float("nan")))
+        ops.attn_prefill(q, kv, outs[-1], table, cu, c, heads, kv_heads, 128, 1 / math.sqrt(128), max(lens), scratch=sc, max_kv_len=longest)
+        _check(outs[-1], q, cu, c, keys, values)
+    assert int(sc.status[0]) == 0
+
+
 @pytest.mark.parametrize("window,softcap,sink", [(1, 0.0, False), (100, 0.0, True), (129, 20.0, False), (0, 30.0, True)])
 def test_masks(window, softcap, sink):
     from llaminar_b200.ops import grouped
