@@ -297,4 +297,80 @@ struct DequantAtomQ4KRt {
     }
 };
 
+// ---- Q5_K to bf16, atom index at run time ------------------------------------------------------------------------------
+// The same idea: a code of five bits, moved to the top of the seven mantissa bits of a bf16 with a zero exponent (two bits to the left),
+// is the subnormal code * 2^-131, so that one HFMA2 with the scale times 2^131 gives scale * code plus the minimum: bit for bit what
+// subtracting a magic offset first gives.  The scaled scale must be finite, |scale| < 1/8 (weights up to 3.9); a warp that meets a
+// larger one takes the way with the offset.  Rotations move the bits, so that one copy of the code serves the four atoms.
+// (Measured in the small-batch GEMM: a step of 13 lanes of a 5-bit 8B model 1388 -> 1326 us.  The same for Q6_K gave nothing there, and in
+// the kernel of CTA pairs either was slower than the way with the offset, 9.0 instead of 8.7 ms for 3 x 700 tokens with routed experts.)
+LLM_DEVICE uint32_t rotl32(uint32_t x, int n) { return __funnelshift_l(x, x, n); }
+LLM_DEVICE __nv_bfloat162 times_2_66(__nv_bfloat162 s, float first) {      // s * first * 2^66 in two exact steps
+    return __hmul2(__hmul2(s, __float2bfloat162_rn(first)), __float2bfloat162_rn(7.3786976e19f));
+}
+// the four codes of a word -> two packed pairs
+template <bool SMALL> LLM_DEVICE void codes_to_bf16(uint32_t w, __nv_bfloat162 off, __nv_bfloat162 s, __nv_bfloat162 b, uint32_t* o) {
+    if (SMALL) {
+        o[0] = hfma2_bf16_u32(__byte_perm(w, 0u, 0x4140), s, b);
+        o[1] = hfma2_bf16_u32(__byte_perm(w, 0u, 0x4342), s, b);
+    } else affine4(w, off, s, b, o[0], o[1]);
+}
+
+struct DequantAtomQ5KRt {
+    struct Regs { uint4 q[2], h[2]; __nv_bfloat162 s_lo, s_hi, b_lo, b_hi; bool small; };
+    LLM_DEVICE static Regs load(uint32_t raw, int g, int lane, int A) {
+        using T = FmtTraits<FMT_Q5_K>;
+        Regs r;
+        const uint32_t qs = raw + unit_off(T::P_QS, 8, g, 2 * A, lane), qh = raw + unit_off(T::P_QH, 2, g, 0, lane);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) { r.q[h] = lds_v4(qs + h * 512); r.h[h] = lds_v4(qh + h * 512); }
+        scales(lds_v4(raw + T::P_META + (((g << 5) + lane) << 4)), A, r);
+        return r;
+    }
+    // 6-bit scales and minima of sub-blocks 2A and 2A + 1 (see DequantAtomQ4KRt)
+    LLM_DEVICE static void scales(const uint4& meta, int A, Regs& r) {
+        const float d = half_bits_to_float(meta.x & 0xffff), ndmin = -half_bits_to_float(meta.x >> 16);
+        const int sh = (A & 1) << 4;
+        const uint32_t a2 = meta.y >> sh, b2 = meta.z >> sh, c2 = meta.w >> sh;
+        uint32_t sc2, mn2;
+        if (A < 2) { sc2 = a2 & 0x3f3fu; mn2 = b2 & 0x3f3fu; }
+        else { sc2 = (c2 & 0x0f0fu) | ((a2 >> 2) & 0x3030u); mn2 = ((c2 >> 4) & 0x0f0fu) | ((b2 >> 2) & 0x3030u); }
+        // byte * f without the conversion unit: the byte under the exponent of 2^23; exact, the product has few bits
+        auto times = [](uint32_t two, uint32_t sel, float f) { return fmaf(__uint_as_float(__byte_perm(two, 0x4b000000u, sel)), f, -8388608.0f * f); };
+        const float s0 = times(sc2, 0x7650, d), s1 = times(sc2, 0x7651, d);
+        r.small = __all_sync(0xffffffffu, fabsf(s0) < 0.1244f && fabsf(s1) < 0.1244f);
+        r.s_lo = __float2bfloat162_rn(s0); r.s_hi = __float2bfloat162_rn(s1);
+        r.b_lo = __float2bfloat162_rn(times(mn2, 0x7650, ndmin)); r.b_hi = __float2bfloat162_rn(times(mn2, 0x7651, ndmin));
+    }
+    template <bool SMALL> LLM_DEVICE static void convert_t(const Regs& r, int A, uint32_t (&o)[32]) {
+        const int r_lo = 6 - 2 * A, r_hi = (5 - 2 * A) & 31;           // bits 2A and 2A + 1 of the high-bit bytes to bit 6
+        const __nv_bfloat162 off = __float2bfloat162_rn(128.0f), quarter = __float2bfloat162_rn(0.25f);
+        const __nv_bfloat162 s_lo = SMALL ? times_2_66(r.s_lo, 3.6893488e19f) : __hmul2(r.s_lo, quarter);
+        const __nv_bfloat162 s_hi = SMALL ? times_2_66(r.s_hi, 3.6893488e19f) : __hmul2(r.s_hi, quarter);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t ws[4] = {r.q[h].x, r.q[h].y, r.q[h].z, r.q[h].w}, hs[4] = {r.h[h].x, r.h[h].y, r.h[h].z, r.h[h].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                codes_to_bf16<SMALL>((rotl32(ws[i], 2) & 0x3c3c3c3cu) | (rotl32(hs[i], r_lo) & 0x40404040u), off, s_lo, r.b_lo, o + 8 * h + 2 * i);
+                codes_to_bf16<SMALL>((rotl32(ws[i], 30) & 0x3c3c3c3cu) | (rotl32(hs[i], r_hi) & 0x40404040u), off, s_hi, r.b_hi, o + 16 + 8 * h + 2 * i);
+            }
+        }
+    }
+    LLM_DEVICE static void convert(const Regs& r, int A, uint32_t (&o)[32]) {
+        if (r.small) convert_t<true>(r, A, o);
+        else convert_t<false>(r, A, o);
+    }
+};
+
+// The formats with a conversion of this kind
+template <int F> struct AtomRt { static constexpr bool HAVE = false; };
+template <> struct AtomRt<FMT_Q4_K> {
+    static constexpr bool HAVE = true;
+    using Regs = DequantAtomQ4KRt::Regs;
+    LLM_DEVICE static Regs load(uint32_t raw, int g, int lane, int A) { return DequantAtomQ4KRt::load(raw, g, lane, A); }
+    LLM_DEVICE static void convert(const Regs& r, int, uint32_t (&o)[32]) { DequantAtomQ4KRt::convert(r, o); }
+};
+template <> struct AtomRt<FMT_Q5_K> : DequantAtomQ5KRt { static constexpr bool HAVE = true; };
+
 }  // namespace llm

@@ -97,8 +97,8 @@ template <int FMT, int BM> struct Cfg {
     static constexpr int A_COLS_OFFSET = 2 * ACC_SET_COLS;
     static constexpr int A_CHUNK_COLS = 128;
     static constexpr int TMEM_COLS = 512;
-    // Q4_K has a conversion with the atom index at run time (one copy of the code for the four warps of a scheduler)
-    static constexpr bool RT_ATOM = (FMT == FMT_Q4_K);
+    // Q4_K and Q5_K have a conversion with the atom index at run time (one copy of the code for the four warps of a scheduler)
+    static constexpr bool RT_ATOM = AtomRt<FMT>::HAVE;
     static_assert(A_COLS_OFFSET + N_SETS * A_CHUNK_COLS <= TMEM_COLS, "tensor memory map overflows");
 };
 
@@ -717,11 +717,12 @@ LLM_DEVICE void gemm_small_body(const CUtensorMap& tmap_x, const GemmTcParams& p
                 if (cc >= C::N_SETS) join();          // from here on an operand set has to be multiplied before it comes free
                 ok = mbar_wait_warp(rawf_bar + slot * 8, rphase, abort_flag);
                 if (LLM_TRACE && warp == 0 && lane == 0) stamp(0, cc * 4 + 0);
-                // Q4_K: the packed bytes and the prepared scales go into registers now, so that the loads and the scale
+                // Q4_K, Q5_K: the packed bytes and the prepared scales go into registers now, so that the loads and the scale
                 // arithmetic run under the wait for the operand slot instead of after it
-                [[maybe_unused]] DequantAtomQ4KRt::Regs pre;
+                using Rt = AtomRt<C::RT_ATOM ? FMT : FMT_Q4_K>;
+                [[maybe_unused]] typename Rt::Regs pre;
                 if constexpr (C::RT_ATOM) {
-                    if (ok) pre = DequantAtomQ4KRt::load(raw_base + slot * C::CHUNK, g, lane, a1);
+                    if (ok) pre = Rt::load(raw_base + slot * C::CHUNK, g, lane, a1);
                 }
                 if (ok) ok = mbar_wait_warp(empty_bar + set * 8, sphase_of(cc) ^ 1, abort_flag);
                 if (LLM_TRACE && warp == 0 && lane == 0) stamp(0, cc * 4 + 1);
@@ -753,7 +754,7 @@ LLM_DEVICE void gemm_small_body(const CUtensorMap& tmap_x, const GemmTcParams& p
                     // chunk ahead of need, so the extra iteration of latency costs nothing.
                     RegSink rs;
                     if constexpr (C::RT_ATOM) {
-                        DequantAtomQ4KRt::convert(pre, rs.o);
+                        Rt::convert(pre, a1, rs.o);
                     } else {
                         switch (a1) {
                             case 0: DequantAtom<FMT, 0>::run(raw, g, lane, rs); break;
