@@ -70,7 +70,7 @@ LLM_DEVICE void quantise_rows(const GemvParams& p, const MoeItem& item, ActBlk* 
         float ss = 0.f;
 #pragma unroll 4
         for (int i = part; i < p.k / 4; i += 128) {
-            const float4 v = x4[i];
+            const float4 v = __ldcg(x4 + i);
             ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         }
         ss = warp_sum(ss);
@@ -82,11 +82,11 @@ LLM_DEVICE void quantise_rows(const GemvParams& p, const MoeItem& item, ActBlk* 
     for (int qd = part; qd < p.k / 4; qd += 128) {          // 4 columns per thread, 8 lanes per 32-column block
         float v0, v1, v2, v3;
         if (NORM) {
-            const float4 v = reinterpret_cast<const float4*>(static_cast<const float*>(p.x) + row)[qd];
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(p.x) + row) + qd);
             const float4 g = reinterpret_cast<const float4*>(p.norm_w)[qd];
             v0 = v.x * rms * g.x; v1 = v.y * rms * g.y; v2 = v.z * rms * g.z; v3 = v.w * rms * g.w;
         } else {
-            const uint2 v = reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.x) + row)[qd];
+            const uint2 v = __ldcg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.x) + row) + qd);
             v0 = bf16_lo(v.x); v1 = bf16_hi(v.x); v2 = bf16_lo(v.y); v3 = bf16_hi(v.y);
         }
         float amax = fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3)));
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(THREADS, 1) moe_stream_kernel(const GemvParams
             bool ok = true;
             while (ok && it.next(u)) {
                 const int item = u.vt / p.n_tiles, tile = u.vt - item * p.n_tiles;
-                const uint8_t* src = p.w + (size_t)p.items[item].expert * p.expert_stride + ((size_t)tile * p.k_blocks + u.kb0) * CHUNK;
+                const uint8_t* src = p.w + (size_t)__ldcg(&p.items[item].expert) * p.expert_stride + ((size_t)tile * p.k_blocks + u.kb0) * CHUNK;
                 for (int c = 0; c < u.nkb && ok; ++c, ++cc) {
                     const int slot = cc % R, phase = (cc / R) & 1;
                     ok = mbar_wait(empty_bar + slot * 8, phase ^ 1, abort_flag);
@@ -174,7 +174,10 @@ __global__ void __launch_bounds__(THREADS, 1) moe_stream_kernel(const GemvParams
             const int item = u.vt / p.n_tiles, tile = u.vt - item * p.n_tiles;
             if (item != cur) {                       // every warp is past the last unit's dot products (barrier below)
                 cur = item;
-                work = p.items[item];
+                // (written by the kernel before, like the rows: L2-coherent loads)
+                work.m = __ldcg(&p.items[item].m);
+#pragma unroll
+                for (int m = 0; m < M; ++m) work.slot[m] = __ldcg(&p.items[item].slot[m]);
                 quantise_rows<NORM>(p, work, acts, s_red + (ui & 1) * (4 * M * 128));
             }
             for (int c = 0; c < u.nkb; ++c, ++cc) {
