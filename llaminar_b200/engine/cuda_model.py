@@ -212,7 +212,7 @@ class QLinear:
 
 def _expert_view_for_tests(pw: PackedWeight, e: int) -> PackedWeight:
     """Expert ``e`` of a packed expert slab as a matrix of its own (tests dequantise it for their fp32 references)."""
-    return PackedWeight(pw.fmt, pw.qtype, pw.n, pw.k, pw.n_tiles, pw.k_blocks, pw.data[e])
+    return PackedWeight(pw.fmt, pw.qtype, pw.n, pw.k, pw.n_tiles, pw.k_blocks, pw.data[e], wide=pw.wide)
 
 
 def _f32(t: QTensor | None, device) -> torch.Tensor | None:

@@ -272,4 +272,4 @@ def moe_forward(model, L, h: torch.Tensor, T: int) -> None:
 
 def _expert_view(pw, e: int):
     from ..ops.layout import PackedWeight
-    return PackedWeight(pw.fmt, pw.qtype, pw.n, pw.k, pw.n_tiles, pw.k_blocks, pw.data[e])
+    return PackedWeight(pw.fmt, pw.qtype, pw.n, pw.k, pw.n_tiles, pw.k_blocks, pw.data[e], wide=pw.wide)

@@ -156,13 +156,16 @@ def moe_combine_sorted(h, y, pos, wts, top_k: int) -> None:
     _count()
 
 
+_WIDE = 4                  # `flags` bit 2: the launcher keeps off the kernels with the short Q4_K conversion
+
+
 def gemm_grouped(pw: PackedWeight, x: torch.Tensor, out: torch.Tensor, row_off: torch.Tensor, tile_off: torch.Tensor, block_m: int, *,
                  epi: int = EPI_STORE, scratch: Scratch | None = None) -> None:
     """Expert GEMMs of one chunk in one launch: rows of ``x`` / ``out`` are sorted by expert, ``row_off`` / ``tile_off``
     (device int32 [experts + 1]) give every expert's first row and first m-tile of height ``block_m``."""
     stride = pw.n_tiles * pw.k_blocks * pw.chunk_bytes
     ext().gemm_tc_grouped(pw.data, pw.fmt, pw.n, pw.k, pw.n_experts, stride, x, out, epi, row_off, tile_off, block_m,
-                          scratch.status if scratch is not None else None)
+                          scratch.status if scratch is not None else None, _WIDE if pw.wide else 0)
     _count()
 
 
@@ -200,7 +203,7 @@ def gemm(pw: PackedWeight, x: torch.Tensor, out: torch.Tensor, *, epi: int = EPI
     if tickets is None and scratch is not None and pw.n_tiles <= scratch.tickets.numel():
         tickets = scratch.tickets          # wider than the split-K accumulator (the LM head): the small-batch kernel needs the counters only
     ext().gemm_tc(pw.data, pw.fmt, pw.n, pw.k, x, out, epi, bias, accum, tickets, ksplit if tickets is not None else 1,
-                  scratch.status if scratch is not None else None, debug_ptr, flags, tp,
+                  scratch.status if scratch is not None else None, debug_ptr, flags | (_WIDE if pw.wide else 0), tp,
                   scratch.partials if scratch is not None else None)
     _count()
 
@@ -212,7 +215,7 @@ def linear_dual(a: PackedWeight, b: PackedWeight, x: torch.Tensor, out_a: torch.
                 norm_w: torch.Tensor | None = None, eps: float = 1e-6, bias_a: torch.Tensor | None = None, bias_b: torch.Tensor | None = None) -> bool:
     """Two matrices of different block formats on the same rows in one launch: the streaming GEMV with ``norm_w`` (up to GEMV_MAX_ROWS
     fp32 rows), the small-batch GEMM without (bf16 rows, up to DUAL_MAX_ROWS).  False, and nothing done, where it does not fit."""
-    if x.shape[0] > (DUAL_MAX_ROWS if norm_w is None else GEMV_MAX_ROWS) or a.k != b.k:
+    if x.shape[0] > (DUAL_MAX_ROWS if norm_w is None else GEMV_MAX_ROWS) or a.k != b.k or a.wide or b.wide:
         return False
     done = ext().linear_dual(a.data, a.fmt, a.n, b.data, b.fmt, b.n, a.k, x, norm_w, eps, out_a, out_b, bias_a, bias_b, scratch.tickets, scratch.partials, scratch.status)
     if done:

@@ -138,7 +138,7 @@ static void moe_combine_sorted(Tensor h, const Tensor& y, const Tensor& pos, con
 
 // Grouped expert GEMM on the tensor cores: rows of x / out sorted by expert (see GemmTcParams::groups in gemm_tc.h).
 static void gemm_tc_grouped(const Tensor& w, int64_t fmt, int64_t n, int64_t k, int64_t groups, int64_t w_group_stride, const Tensor& x, Tensor out,
-                            int64_t epi, const Tensor& row_off, const Tensor& tile_off, int64_t bm, const OptTensor& status) {
+                            int64_t epi, const Tensor& row_off, const Tensor& tile_off, int64_t bm, const OptTensor& status, int64_t flags) {
     check_cuda(w, "w"); check_cuda(x, "x"); check_cuda(out, "out");
     const c10::cuda::CUDAGuard guard(x.device());
     TORCH_CHECK(x.scalar_type() == torch::kBFloat16 && x.is_contiguous(), "grouped GEMM input must be contiguous bf16");
@@ -150,7 +150,7 @@ static void gemm_tc_grouped(const Tensor& w, int64_t fmt, int64_t n, int64_t k, 
     p.x = static_cast<const __nv_bfloat16*>(x.data_ptr());
     p.out = out.data_ptr(); p.out_stride = (int)out.stride(0); p.out_f32 = out.scalar_type() == torch::kFloat32;
     TORCH_CHECK(out.size(0) >= x.size(0), "grouped GEMM: out has fewer rows than x");
-    p.epi = (int)epi; p.status = mptr<int>(status); p.ksplit = 1;
+    p.epi = (int)epi; p.status = mptr<int>(status); p.ksplit = 1; p.flags = (int)flags;
     p.groups = (int)groups; p.w_group_stride = (long long)w_group_stride; p.group_bm = (int)bm;
     p.group_row_off = static_cast<const int*>(row_off.data_ptr()); p.group_tile_off = static_cast<const int*>(tile_off.data_ptr());
     LLM_CUDA_CHECK(llm::launch_gemm_tc(p, cur_stream()));

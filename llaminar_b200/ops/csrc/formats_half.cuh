@@ -2,7 +2,8 @@
 // row (lane == row inside the 32-row group g), for the warps that feed tensor memory.
 //     Regs r = HalfChunk<FMT>::load(chunk, g, lane, H)       the packed bytes, from global memory
 //     HalfChunk<FMT>::atom<K>(r, H, o, grid)                 atom 2H + K: 64 bf16 as 32 packed pairs, columns in order
-// H is the same in all lanes.  Values are those of DequantBlock (formats.cuh), bit for bit.
+// H is the same in all lanes.  Values are those of DequantBlock (formats.cuh), bit for bit; Q4_K for scales below 0.5 (DequantAtomQ4KRt:
+// GEMMs of matrices with larger ones do not come here).
 #pragma once
 #include "formats_smem.cuh"
 

@@ -232,8 +232,9 @@ template <int A> struct DequantAtom<FMT_IQ3_S, A> {
 // times 2^129 and its (negated) minimum then yields two weights with a single rounding: bit for bit what
 // (128 + q - 128) * scale - min gives, for one half2 operation less per pair.  Per 8 weights: 3 logic ops, 4 byte permutes,
 // 4 HFMA2 (the generic path spends 3 + 4 + 8).  The scale times 2^129 must stay finite in bf16, i.e. d * sc < 0.5 (weights
-// up to about +-7); larger scales are clamped to the largest finite value, and the loader re-encodes such a tensor instead
-// of sending it here (ops/layout.py: q4k_scales_in_range).
+// up to about +-7); larger scales are clamped to the largest finite value, and matrices that have them are marked when they are
+// packed and stay on the large-tile GEMM (ops/layout.py: q4k_scales_in_range).  (Choosing the way with the offset by a warp vote
+// here instead cost the steps of 4-bit models 2 to 4 %.)
 // The atom index is a run-time value so that the four warps of a scheduler (same row group, different atoms) share one
 // copy of the code.  The sink receives the whole atom at once: sink.emit64(r) -> the 64 columns of atom A of this lane's row.
 // (A fp16 variant through cvt.rn.f16x2.e4m3x2 was tried first: tcgen05.mma kind::f16 with an fp16 A and a bf16 B operand

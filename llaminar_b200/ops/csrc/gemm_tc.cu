@@ -620,6 +620,9 @@ cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st) {
     if (p.k % 256 || (reinterpret_cast<uintptr_t>(xa) & 15)) return cudaErrorInvalidValue;
     int bm, ks;
     gemm_tc_plan(p.m, p.n, p.k, p.ksplit, &bm, &ks);
+    const bool wide = p.flags & GEMM_WIDE;         // everything below keeps it on the kernel here
+    if (wide && p.tp) return cudaErrorInvalidValue;   // the fused all-reduce lives in the small-batch kernel
+    if (wide && bm == 32) bm = 64;
     if (p.ag_on) {
         if (p.m <= 32) bm = 64;                    // the fused all-gather lives in the large-tile kernel
         if (p.ag.world < 1 || p.ag.world > 8 || p.ag.copy_ctas < 1 || p.ag.rows_per_rank < 1) return cudaErrorInvalidValue;
@@ -638,16 +641,16 @@ cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st) {
         ks = 1;
     }
     if (ks > 1 && (!p.accum || !p.tickets)) ks = 1;
-    if (bm <= 128 && !p.rs_on && !p.ag_on && p.groups == 0) {
+    if (bm <= 128 && !p.rs_on && !p.ag_on && p.groups == 0 && !wide) {
         // Up to 128 rows the product is a stream of weights: the persistent kernel reads it once, every SM the same share.  It
         // wants the chunks on 16-byte boundaries and work indices of 32 bits; calls of 33 rows or more without these keep
         // the kernel of large tiles, as they always had it.
         const bool fits = !(reinterpret_cast<uintptr_t>(p.w) & 15) && ((unsigned long long)((p.n + 127) / 128) * (p.k / 256) + 1) * 148ull < (1ull << 32);
         if (bm == 32 || (fits && !p.tp)) return launch_gemm_tc_small(p, bm, (p.tickets && p.ksplit != 1) ? 0 : 1, st);
     }
-    // More rows, and the groups of expert GEMMs, run on pairs of CTAs; the kernel here keeps the fused collectives, forced splits, traces
-    // and more groups than the pairs keep offsets for.
-    if (!p.rs_on && !p.ag_on && !p.debug && p.groups <= 256) {
+    // More rows, and the groups of expert GEMMs, run on pairs of CTAs; the kernel here keeps the fused collectives, forced splits, traces,
+    // Q4_K scales that the short conversion does not take, and more groups than the pairs keep offsets for.
+    if (!p.rs_on && !p.ag_on && !p.debug && p.groups <= 256 && !wide) {
         if (p.groups > 0) return launch_gemm_tc_pair(p, bm, st);
         // (up to 256 rows of a narrow and long matrix leave most pairs without a tile: there this kernel splits K instead.
         // 5120 x 25600 Q4_K, 160 rows: 99 us here, 124 us there; 4096 x 12288: 62 and 63 us.)

@@ -42,6 +42,8 @@ struct RsFuse {
     int flags_per_parity;
 };
 
+constexpr int GEMM_WIDE = 4;
+
 struct GemmTcParams {
     const uint8_t* w;          // weight chunks [n_tiles][k_blocks][chunk]
     int fmt;
@@ -60,7 +62,8 @@ struct GemmTcParams {
     int* status;               // optional device word: set to STATUS_TIMEOUT if a pipeline wait gave up
     int* debug;                // optional trace buffer (progress markers / ns timestamps written by the kernels); nullptr in production
     const TpFuse* tp;          // EPI_RESID in the small-batch kernel: fused cross-rank all-reduce of each tile (nullptr: off)
-    int flags;                 // bit 1 (set by the launcher): stream-K work split in the small-batch kernel; with `debug`: 0x100 makes the
+    int flags;                 // bit 1 (set by the launcher): stream-K work split in the small-batch kernel; bit 2 (GEMM_WIDE): Q4_K scales
+                               // that only the large-tile kernel converts; with `debug`: 0x100 makes the
                                // large-tile kernel write per-CTA ns timestamps (8 x u64 per CTA) instead of progress markers, bits 8.. select
                                // the traced CTA of the small-batch kernel
     int ag_on;                 // large-tile kernel: x rows are gathered from the ranks of `ag` inside the launch

@@ -55,6 +55,7 @@ class PackedWeight:
     k_blocks: int
     data: torch.Tensor          # uint8 [experts?][n_tiles * k_blocks * chunk_bytes]
     n_experts: int = 0
+    wide: bool = False          # Q4_K scales beyond the short conversion's range (`q4k_scales_in_range`): GEMMs take the exact, slower one
 
     @property
     def chunk_bytes(self) -> int:
@@ -78,13 +79,14 @@ def _planes_of(qtype: GGMLType, blocks: torch.Tensor) -> list[torch.Tensor]:
     raise NotImplementedError(qtype)
 
 
-Q4K_MAX_D = 0.5 / 63          # the small-batch GEMM multiplies d * sc by 2^129 in bf16: d * sc must stay below 0.5
+Q4K_MAX_D = 0.5 / 63          # the short conversion multiplies d * sc by 2^129 in bf16: d * sc must stay below 0.5
 
 
 def q4k_scales_in_range(raw: torch.Tensor) -> bool:
-    """Whether every super-block scale ``d`` of a Q4_K tensor is small enough for the small-batch GEMM's conversion
-    (csrc/formats_smem.cuh: DequantAtomQ4KRt).  Real checkpoints are two orders of magnitude below the limit (it allows
-    weights up to about +-7); a tensor that is not gets re-encoded by the loader instead of silently losing range."""
+    """Whether every super-block scale ``d`` of a Q4_K tensor is small enough for the short conversion of the small-batch and the
+    pair GEMM (csrc/formats_smem.cuh: DequantAtomQ4KRt).  Real checkpoints are two orders of magnitude below the limit (it
+    allows weights up to about +-7).  A dense matrix that is not is re-encoded by the loader; packed matrices and expert stacks
+    carry it as ``PackedWeight.wide``, and their GEMMs run on the large-tile kernel, whose conversion has no limit."""
     d = raw.reshape(-1, 144)[:, :2].contiguous().view(torch.float16).float().abs()
     d = torch.nan_to_num(d, nan=float("inf"))
     return bool((d.max() <= Q4K_MAX_D).item()) if d.numel() else True
@@ -96,7 +98,11 @@ def can_pack(qtype: GGMLType, k: int) -> bool:
 
 def pack_matrix(raw: torch.Tensor, qtype: GGMLType, n: int, k: int) -> PackedWeight:
     """raw: flat uint8 GGUF bytes of W[n, k] (row-major blocks) -> chunk layout (same device)."""
-    qtype = GGMLType(qtype)
+    wide = qtype == GGMLType.Q4_K and not q4k_scales_in_range(raw)
+    return _pack(raw, GGMLType(qtype), n, k, wide)
+
+
+def _pack(raw: torch.Tensor, qtype: GGMLType, n: int, k: int, wide: bool) -> PackedWeight:
     if not can_pack(qtype, k):
         raise ValueError(f"cannot tile {qtype.name} with k={k}")
     e, b = BLOCK_GEOMETRY[qtype]
@@ -117,15 +123,16 @@ def pack_matrix(raw: torch.Tensor, qtype: GGMLType, n: int, k: int) -> PackedWei
         outs.append(p.reshape(nt, kb, TILE_N * r))
     data = torch.cat(outs, dim=2).contiguous().reshape(-1)
     assert data.numel() == nt * kb * chunk_bytes(qtype)
-    return PackedWeight(FMT_IDS[qtype], qtype, n, k, nt, kb, data)
+    return PackedWeight(FMT_IDS[qtype], qtype, n, k, nt, kb, data, wide=wide)
 
 
 def pack_experts(raw: torch.Tensor, qtype: GGMLType, n_experts: int, n: int, k: int) -> PackedWeight:
     per = raw.numel() // n_experts
-    parts = [pack_matrix(raw[e * per:(e + 1) * per], qtype, n, k) for e in range(n_experts)]
+    wide = qtype == GGMLType.Q4_K and not q4k_scales_in_range(raw)
+    parts = [_pack(raw[e * per:(e + 1) * per], GGMLType(qtype), n, k, wide) for e in range(n_experts)]
     p0 = parts[0]
     data = torch.stack([p.data for p in parts])
-    return PackedWeight(p0.fmt, p0.qtype, n, k, p0.n_tiles, p0.k_blocks, data, n_experts)
+    return PackedWeight(p0.fmt, p0.qtype, n, k, p0.n_tiles, p0.k_blocks, data, n_experts, wide)
 
 
 def concat_rows(parts: list[tuple[torch.Tensor, GGMLType, int, int]]) -> tuple[torch.Tensor, GGMLType, int, int]:
