@@ -50,6 +50,49 @@ constexpr uint32_t IDESC_S = instr_desc(BK), IDESC_O = instr_desc(D) | (1u << 16
 LLM_DEVICE void cp_async16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
 LLM_DEVICE void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// One row's attention over keys [k0, k1) alone, by a warp: lane i has values 4i .. 4i + 3 of q and of the unscaled result o.
+// `row_of(key, kv)`: the key's K (0) or V (1) row.
+template <bool CAP, class F>
+LLM_DEVICE void exact_row(const __nv_bfloat16* q, int k0, int k1, const ScoreScale& score, F&& row_of, float& m, float& l, float (&o)[4]) {
+    const int lane = threadIdx.x & 31;
+    auto four = [&](const __nv_bfloat16* x, float (&f)[4]) {
+        const uint2 v = __ldcg(reinterpret_cast<const uint2*>(x + lane * 4));
+        f[0] = bf16_lo(v.x); f[1] = bf16_hi(v.x); f[2] = bf16_lo(v.y); f[3] = bf16_hi(v.y);
+    };
+    float a[4];
+    four(q, a);
+    m = -INFINITY; l = 0.f;
+    o[0] = o[1] = o[2] = o[3] = 0.f;
+#pragma unroll 4
+    for (int key = k0; key < k1; ++key) {
+        float k[4], v[4];
+        four(row_of(key, 0), k);
+        four(row_of(key, 1), v);
+        const float s = warp_sum(a[0] * k[0] + a[1] * k[1] + a[2] * k[2] + a[3] * k[3]);
+        const float x = CAP ? score.capped(s) : score.linear(s), top = fmaxf(m, x);
+        if (top == -INFINITY) continue;                    // a score of -inf: probability 0
+        const float c = exp2f(m - top), e = exp2f(x - top);
+        m = top;
+        l = l * c + e;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = o[i] * c + e * v[i];
+    }
+}
+
+// Four values a lane of a row's unscaled result, on to the output: the sink's share of the denominator, the output gate
+LLM_DEVICE void finish_row(const AttnPrefillParams& p, size_t at, int head, float m, float l, float (&o)[4]) {
+    const int lane = threadIdx.x & 31;
+    if (p.sink) l += exp2f(p.sink[head] * LOG2E - m);
+    float inv = l > 0.f ? 1.f / l : 0.f;
+    if (p.gate && p.gate_heads) inv *= __fdividef(1.f, 1.f + __expf(-__bfloat162float(p.gate[at * p.gate_row + head])));
+    if (p.gate && !p.gate_heads) {
+        const uint2 g = *reinterpret_cast<const uint2*>(p.gate + at * p.gate_row + head * D + lane * 4);
+        o[0] *= __fdividef(1.f, 1.f + __expf(-bf16_lo(g.x))); o[1] *= __fdividef(1.f, 1.f + __expf(-bf16_hi(g.x)));
+        o[2] *= __fdividef(1.f, 1.f + __expf(-bf16_lo(g.y))); o[3] *= __fdividef(1.f, 1.f + __expf(-bf16_hi(g.y)));
+    }
+    *reinterpret_cast<uint2*>(p.out + (at * p.n_heads + head) * D + lane * 4) = make_uint2(pack_bf16(o[0] * inv, o[1] * inv), pack_bf16(o[2] * inv, o[3] * inv));
+}
+
 enum Bar { K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, Q_FULL = 8, S_FULL = 9, P_FULL = 11, O_FULL = 13, N_BARS = 15 };
 
 template <bool CAP>                                // scores are soft-capped
@@ -200,6 +243,8 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
                 mbar_arrive_if(bar(P_FULL + slot), lane == 0);
             }
             ok = ok && mbar_wait_warp(bar(O_FULL + slot), 0, abort_flag);
+            const float sum_l = l;
+            float odd = 0.f;                                       // NaN once a value of the row's O is not finite
             if (ok && splits > 1) {
                 tc_fence_after();
                 const size_t at = part + (size_t)slot * splits * BQ + row;
@@ -208,6 +253,8 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
                 for (int c = 0; c < 4; ++c) {
                     uint32_t r[32];
                     tmem_ld_n<32>(t_o + c * 32, r);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) odd = fmaf(__uint_as_float(r[i]), 0.f, odd);
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
                         dst[c * 8 + u] = make_float4(__uint_as_float(r[4 * u]), __uint_as_float(r[4 * u + 1]), __uint_as_float(r[4 * u + 2]), __uint_as_float(r[4 * u + 3]));
@@ -225,6 +272,8 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
                 for (int c = 0; c < 4; ++c) {
                     uint32_t r[32];
                     tmem_ld_n<32>(t_o + c * 32, r);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) odd = fmaf(__uint_as_float(r[i]), 0.f, odd);
                     if (row < rows) {
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
@@ -247,6 +296,36 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
                         }
                     }
                 }
+            }
+            // A masked key has P = 0, and 0 times an infinity or NaN in its V row (a later token, or what the page held before) is
+            // NaN.  Rows that are not finite although their scores are, and that have such a key in their tiles, are computed again
+            // over their own keys alone.
+            unsigned again = __ballot_sync(0xffffffffu, ok && row < rows && odd != 0.f && fabsf(sum_l) <= 3.4e38f);
+            if (again) __syncwarp();                               // the stores above come before the ones below
+#pragma unroll 1
+            for (; again; again &= again - 1) {
+                const int src = __ffs(again) - 1, i = (warp & 3) * 32 + src;
+                const int t0 = tile0 * BK, t1 = t0 + nt * BK, k0 = max(t0, __shfl_sync(0xffffffffu, low, src)), k1 = max(k0, min(t1, __shfl_sync(0xffffffffu, lim, src)));
+                auto row_of = [&](int key, int kv) {
+                    const size_t page = LLM_CHECK_INDEX(btab[min(key / PAGE, n_pages - 1)], p.n_pages);
+                    return p.kv + (((page * 2 + kv) * p.n_kv_heads + kvh) * PAGE + key % PAGE) * D;
+                };
+                float zero = 0.f;
+#pragma unroll 1
+                for (int key = t0; key < t1; ++key) {
+                    if (key == k0) { key = k1; if (key >= t1) break; }
+                    const uint2 v = __ldcg(reinterpret_cast<const uint2*>(row_of(key, 1) + lane * 4));
+                    zero += (bf16_lo(v.x) + bf16_hi(v.x)) * 0.f + (bf16_lo(v.y) + bf16_hi(v.y)) * 0.f;
+                }
+                if (!__any_sync(0xffffffffu, zero != 0.f)) continue;
+                const size_t at = (size_t)(q_start + q0 + i);
+                float rm, rl, o[4];
+                exact_row<CAP>(p.q + (at * p.n_heads + head) * D, k0, k1, score, row_of, rm, rl, o);
+                if (splits > 1) {
+                    const size_t mine = part + (size_t)slot * splits * BQ + i;
+                    *reinterpret_cast<float4*>(p.part_o + mine * D + lane * 4) = make_float4(o[0], o[1], o[2], o[3]);
+                    if (lane == 0) *reinterpret_cast<float2*>(p.part_ml + mine * 2) = make_float2(rm, rl);
+                } else finish_row(p, at, head, rm, rl, o);
             }
         }
     } else {
@@ -342,16 +421,7 @@ __global__ void __launch_bounds__(128) paged_attn_prefill_merge_kernel(const Att
         l += c * ml.y;
         o[0] += c * v.x; o[1] += c * v.y; o[2] += c * v.z; o[3] += c * v.w;
     }
-    const size_t at = (size_t)(q_start + r);
-    if (p.sink) l += exp2f(p.sink[head] * LOG2E - m);
-    float inv = l > 0.f ? 1.f / l : 0.f;
-    if (p.gate && p.gate_heads) inv *= __fdividef(1.f, 1.f + __expf(-__bfloat162float(p.gate[at * p.gate_row + head])));
-    if (p.gate && !p.gate_heads) {
-        const uint2 g = *reinterpret_cast<const uint2*>(p.gate + at * p.gate_row + head * D + lane * 4);
-        o[0] *= __fdividef(1.f, 1.f + __expf(-bf16_lo(g.x))); o[1] *= __fdividef(1.f, 1.f + __expf(-bf16_hi(g.x)));
-        o[2] *= __fdividef(1.f, 1.f + __expf(-bf16_lo(g.y))); o[3] *= __fdividef(1.f, 1.f + __expf(-bf16_hi(g.y)));
-    }
-    *reinterpret_cast<uint2*>(p.out + (at * p.n_heads + head) * D + lane * 4) = make_uint2(pack_bf16(o[0] * inv, o[1] * inv), pack_bf16(o[2] * inv, o[3] * inv));
+    finish_row(p, (size_t)(q_start + r), head, m, l, o);
 }
 
 static int pairs_of(int n_heads, int n_kv_heads, int max_q_len) { return ((max_q_len + BQ - 1) / BQ * (n_heads / n_kv_heads) + 1) / 2; }

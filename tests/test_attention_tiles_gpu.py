@@ -93,3 +93,37 @@ def test_masks(window, softcap, sink):
     grouped.attn_prefill(q, kv, out, table, cu, c, 1 / math.sqrt(128), max(lens), window, logits, None, status, softcap=softcap)
     assert int(status[0]) == 0
     _check(out, q, cu, c, keys, values, window=window, softcap=softcap, sink=logits)
+
+
+@pytest.mark.parametrize("window,softcap", [(0, 0.0), (100, 20.0)])
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+@pytest.mark.parametrize("heads,kv_heads,lens,ctx,late", [(8, 2, [200, 64, 1], [0, 100, 63], 130), (7, 1, [140, 300], [200, 0], 60), (4, 4, [17, 250], [513, 0], 9), (32, 8, [40], [2000], 30)])
+def test_values_behind_the_mask(heads, kv_heads, lens, ctx, late, bad, window, softcap):
+    """V rows that are not finite, of a later token and in what a page held before, reach no row that does not see them; rows that do
+    are not finite in those columns and right in the others."""
+    from llaminar_b200 import ops
+    from llaminar_b200.ops import grouped
+    q, kv, table, cu, c, keys, values = _case(heads, kv_heads, lens, ctx, False, 3)
+    for b, (n, m) in enumerate(zip(lens, ctx)):
+        end = n + m
+        if end % 64:
+            kv[table[b, end // 64], 1, :, end % 64:] = bad
+        kv[table[b, end // 64 + 1], 1] = bad
+        if n > late:
+            at = m + late
+            kv[table[b, at // 64], 1, :, at % 64, 5:9] = bad
+            values[b][at, :, 5:9] = 0
+    out, sc = torch.full_like(q, 7.0), ops.scratch_for(DEV)
+    if window or softcap:
+        grouped.attn_prefill(q, kv, out, table, cu, c, 1 / math.sqrt(128), max(lens), window, None, None, sc.status, softcap=softcap)
+    else:
+        ops.attn_prefill(q, kv, out, table, cu, c, heads, kv_heads, 128, 1 / math.sqrt(128), max(lens), tensor_core=True, scratch=sc, max_kv_len=max(n + m for n, m in zip(lens, ctx)))
+    assert int(sc.status[0]) == 0
+    for b, (k, v) in enumerate(zip(keys, values)):
+        rows = slice(int(cu[b]), int(cu[b + 1]))
+        want, got = _reference(q[rows], k, v, int(ctx[b]), window=window, softcap=softcap), out[rows].double()
+        place = torch.arange(lens[b], device=DEV)
+        sees = (place >= late) & ((place < late + window) if window else (place >= 0)) if lens[b] > late else torch.zeros_like(place, dtype=torch.bool)
+        assert not bool(got[sees][..., 5:9].isfinite().any())
+        got[sees.nonzero()[:, 0], :, 5:9] = want[sees.nonzero()[:, 0], :, 5:9]
+        assert (got - want).norm() <= REL * want.norm(), b
