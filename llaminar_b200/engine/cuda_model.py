@@ -164,7 +164,7 @@ class QLinear:
             qt = group[0].qtype
             raw = torch.cat([q.raw.to(device).reshape(-1) for q in group]) if len(group) > 1 else group[0].raw.to(device)
             if can_pack(qt, k):
-                parts.append((pack_matrix(raw, qt, n, k), col))          # rows are padded to whole 128-row tiles
+                parts.append((pack_matrix(raw, qt, n, k, in_range=True), col))          # rows are padded to whole 128-row tiles
             else:
                 from ..gguf import dequantize
                 parts.append((dequantize(raw, qt, (n, k)).to(torch.bfloat16), col))
@@ -384,7 +384,7 @@ class CudaModel:
         t = for_kernels(t)
         n, k = t.shape
         if can_pack(t.qtype, k):
-            return pack_matrix(t.raw.to(self.device), t.qtype, n, k)
+            return pack_matrix(t.raw.to(self.device), t.qtype, n, k, in_range=True)
         return t.to_float().to(self.device)
 
     def _build_layer(self, w: ModelWeights, i: int) -> CudaLayer:
@@ -467,7 +467,7 @@ class CudaModel:
         n, k = g.shape
         if g.qtype == u.qtype and can_pack(g.qtype, k) and n % 16 == 0:
             raw, qt, n2, _ = interleave_gate_up(g.raw.to(dev), u.raw.to(dev), g.qtype, n, k)
-            lin = QLinear([(pack_matrix(raw, qt, n2, k), 0)], n2, k)
+            lin = QLinear([(pack_matrix(raw, qt, n2, k, in_range=True), 0)], n2, k)
             lin.fused_swiglu = True
             return lin
         lin = QLinear.from_qtensors([g, u], dev)

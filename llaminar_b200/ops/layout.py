@@ -96,9 +96,10 @@ def can_pack(qtype: GGMLType, k: int) -> bool:
     return qtype in FMT_IDS and k % TILE_K == 0
 
 
-def pack_matrix(raw: torch.Tensor, qtype: GGMLType, n: int, k: int) -> PackedWeight:
-    """raw: flat uint8 GGUF bytes of W[n, k] (row-major blocks) -> chunk layout (same device)."""
-    wide = qtype == GGMLType.Q4_K and not q4k_scales_in_range(raw)
+def pack_matrix(raw: torch.Tensor, qtype: GGMLType, n: int, k: int, in_range: bool = False) -> PackedWeight:
+    """raw: flat uint8 GGUF bytes of W[n, k] (row-major blocks) -> chunk layout (same device).  ``in_range``: the caller has looked
+    at the scales of a Q4_K matrix already (here that is a reduction and a synchronisation)."""
+    wide = not in_range and qtype == GGMLType.Q4_K and not q4k_scales_in_range(raw)
     return _pack(raw, GGMLType(qtype), n, k, wide)
 
 
