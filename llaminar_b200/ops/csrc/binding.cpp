@@ -683,6 +683,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("gemm_tc_grouped", &gemm_tc_grouped);
     m.def("gemm_tc", &gemm_tc);
     m.def("linear_dual", &linear_dual);
+    m.def("share_ctas", [](double bytes_a, double bytes_b, int most_a, int most_b, int ctas) {
+        const llm::Shares s = llm::share_ctas(bytes_a, bytes_b, most_a, most_b, ctas);
+        return std::make_pair(s.first, s.second);
+    });
     m.def("gemm_tc_allgather", &gemm_tc_allgather);
     m.def("gemm_tc_rs", &gemm_tc_rs);
     m.def("rs_reduce_norm", &rs_reduce_norm);

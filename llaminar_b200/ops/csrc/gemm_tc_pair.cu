@@ -329,12 +329,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_pair_kernel(const __grid_cons
     if (warp == DEQUANT_WARPS + 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-static int sm_count() {
-    static int n = 0;
-    if (!n) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); }
-    return n > 1 ? n : 148;
-}
-
 template <int FMT>
 static cudaError_t launch_one(const GemmTcParams& p, int bt, cudaStream_t st) {
     static bool attr_set = false;
@@ -364,7 +358,7 @@ static cudaError_t launch_one(const GemmTcParams& p, int bt, cudaStream_t st) {
 // MMAs (1.5 us with 256 tokens) or as its conversion (1.1 us from Q4_K and Q4_0, 1.4 us from the others), whichever is longer, a tile
 // some of that time more for its start and end.
 int gemm_pair_tokens(int fmt, int m, int n, int k) {
-    const int pairs = ((n + 127) / 128 + 1) / 2, kb = k / 256, slots = tcp::sm_count() / 2;
+    const int pairs = ((n + 127) / 128 + 1) / 2, kb = k / 256, slots = sm_count() / 2;
     const double least_chunk = fmt == FMT_Q4_K || fmt == FMT_Q4_0 ? 0.7 : 0.9;
     int best = 256;
     double least = 0.;

@@ -962,9 +962,7 @@ static cudaError_t launch_one(const GemmTcParams& p, int ksplit, cudaStream_t st
     const bool streamk = ksplit != 1 && p.tickets && (p.partials || (p.accum && !C::WIDE));
     q.flags = (p.flags & ~2) | (streamk ? 2 : 0);
     const int units = streamk ? n_tiles * k_blocks : n_tiles;
-    static int cached_sms = 0;
-    if (!cached_sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&cached_sms, cudaDevAttrMultiProcessorCount, dev); }
-    const int sms = cached_sms > 0 ? cached_sms : 148;
+    const int sms = sm_count();
     int grid = units < sms ? units : sms;
     if (streamk) {
         // small problems: at least four chunks per CTA (the per-CTA start-up and epilogue cost a few chunks' worth of
@@ -1005,12 +1003,8 @@ static cudaError_t launch_dual(const GemmTcParams& a, const GemmTcParams& b, cud
     const int kb = a.k / 256, ta = (a.n + 127) / 128, tb = (b.n + 127) / 128;
     auto most = [&](int tiles) { const int g1 = (tiles * kb + 3) / 4, g2 = 4 * tiles; return g1 < g2 ? g1 : g2; };
     const double wa = (double)ta * Cfg<FA, BM>::CHUNK, wb = (double)tb * Cfg<FB, BM>::CHUNK;
-    int gb = (int)(148 * wb / (wa + wb) + 0.5);
-    if (gb > most(tb)) gb = most(tb);
-    if (gb < 1) gb = 1;
-    int ga = 148 - gb;
-    if (ga > most(ta)) ga = most(ta);
-    if (ga < 1 || gb > 147) return cudaErrorNotSupported;
+    const auto [ga, gb] = share_ctas(wa, wb, most(ta), most(tb), sm_count() < 148 ? sm_count() : 148);      // (slots for 148 CTAs)
+    if (!ga) return cudaErrorNotSupported;
     if ((unsigned long long)((long long)(ta > tb ? ta : tb) * kb + 1) * 148ull >= (1ull << 32)) return cudaErrorNotSupported;       // 32-bit work indices
     GemmTcParams qa = a, qb = b;
     qa.flags = qb.flags = 2;                         // split tiles

@@ -392,12 +392,8 @@ static cudaError_t launch_dual(const GemvParams& a, const GemvParams& b, int m, 
     // CTAs by bytes, at least four chunks per CTA, as for one matrix
     const int ca = a.n_tiles * a.k_blocks, cb = b.n_tiles * b.k_blocks;
     const double wa = (double)ca * FmtTraits<FA>::CHUNK, wb = (double)cb * FmtTraits<FB>::CHUNK;
-    int gb = (int)(148 * wb / (wa + wb) + 0.5);
-    if (gb > cb / 4) gb = cb / 4;
-    if (gb < 1) gb = 1;
-    int ga = 148 - gb;
-    if (ga > ca / 4) ga = ca / 4;
-    if (ga < 1) ga = 1;
+    const auto [ga, gb] = share_ctas(wa, wb, ca / 4, cb / 4, sm_count() < 148 ? sm_count() : 148);      // (slots for 148 CTAs)
+    if (!ga) return cudaErrorNotSupported;
     size_t sa = 0, sb = 0;
     const Extra ea = ring<FA>(a, m, (ca + ga - 1) / ga + 1, partials, tickets, status, &sa);
     const Extra eb = ring<FB>(b, m, (cb + gb - 1) / gb + 1, partials + (size_t)ga * 4 * 128, tickets + a.n_tiles, status, &sb);
@@ -434,9 +430,7 @@ cudaError_t launch_gemv_stream(const GemvParams& p, int m, float* partials, size
     if (reinterpret_cast<uintptr_t>(p.w) & 15) return cudaErrorNotSupported;
     const int total = p.n_tiles * p.k_blocks;
     if ((unsigned long long)((long long)total + 1) * 148ull >= (1ull << 32)) return cudaErrorNotSupported;      // 32-bit work indices
-    static int cached_sms = 0;
-    if (!cached_sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&cached_sms, cudaDevAttrMultiProcessorCount, dev); }
-    const int sms = cached_sms > 0 ? cached_sms : 148;
+    const int sms = sm_count();
     int grid = total / 4;                       // at least four chunks per CTA: the start-up and the epilogue cost a few chunks' time
     if (grid > sms) grid = sms;
     if (grid < 1) grid = 1;

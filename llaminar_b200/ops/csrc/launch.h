@@ -14,6 +14,28 @@
 
 namespace llm {
 
+// SMs of the current device.  CTAs of the persistent kernels wait for one another, so a launch has no more of them than fit at once.
+inline int sm_count() {
+    static int n = 0;
+    if (!n) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); }
+    return n > 0 ? n : 148;
+}
+
+// CTAs of two matrices that share a launch of `ctas` in all: by bytes, no more than `most` of either and at least one.
+// {0, 0}: there is no room for two.
+struct Shares { int first, second; };
+inline Shares share_ctas(double bytes_a, double bytes_b, int most_a, int most_b, int ctas) {
+    if (ctas < 2) return {0, 0};
+    int b = (int)(ctas * bytes_b / (bytes_a + bytes_b) + 0.5);
+    if (b > most_b) b = most_b;
+    if (b > ctas - 1) b = ctas - 1;
+    if (b < 1) b = 1;
+    int a = ctas - b;
+    if (a > most_a) a = most_a;
+    if (a < 1) a = 1;
+    return {a, b};
+}
+
 inline bool& pdl_enabled() {
     static bool on = true;
     return on;

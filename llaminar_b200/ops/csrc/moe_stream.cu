@@ -320,9 +320,7 @@ cudaError_t launch_moe_stream(const GemvParams& p, int z_max, float* partials, s
     if (p.norm_w ? ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.norm_w)) & 15) || p.x_stride % 4 : (reinterpret_cast<uintptr_t>(p.x) & 7) || p.x_stride % 4)
         return cudaErrorNotSupported;
     const unsigned long long units = (unsigned long long)z_max * p.n_tiles;
-    static int cached_sms = 0;
-    if (!cached_sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&cached_sms, cudaDevAttrMultiProcessorCount, dev); }
-    const int grid = cached_sms > 0 ? cached_sms : 148;
+    const int grid = sm_count();
     if (units > n_tickets || (units * p.k_blocks + 1) * grid >= (1ull << 32) || (size_t)grid * ms::M * 128 > partials_floats) return cudaErrorNotSupported;
     const ms::Extra e{partials, tickets, status, 0};
     cudaError_t err = cudaErrorInvalidValue;

@@ -14,9 +14,9 @@ def _rel(a, b):
 
 @pytest.mark.parametrize("fa,fb", [(GGMLType.Q4_K, GGMLType.Q6_K), (GGMLType.Q4_K, GGMLType.Q5_K), (GGMLType.Q5_K, GGMLType.Q6_K)])
 @pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 32, 33, 64, 100, 128])
-@pytest.mark.parametrize("na,nb,k", [(256, 128, 256), (200, 100, 768), (5120, 1024, 2048), (128, 4096, 1024)])
+@pytest.mark.parametrize("na,nb,k", [(256, 128, 256), (200, 100, 768), (5120, 1024, 2048), (128, 4096, 1024), (128, 128 * 500, 1024)])
 def test_dual(fa, fb, rows, na, nb, k):
-    """A tile or less each, more CTAs than chunks, ragged columns, the second matrix the larger one."""
+    """A tile or less each, more CTAs than chunks, ragged columns, the second matrix the larger one, and all but a five hundredth."""
     from llaminar_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(rows)
     raw = [quantize(torch.randn(n, k, device=DEV, generator=g) * 0.05, f) for n, f in ((na, fa), (nb, fb))]
