@@ -972,9 +972,7 @@ static cudaError_t launch_one(const GemmTcParams& p, int ksplit, cudaStream_t st
         if (g < 1) g = 1;
         if (g < grid) grid = g;
     }
-    if (grid > 148) {                                // the slot workspace is sized for 148 CTAs
-        if (C::WIDE) grid = 148; else q.partials = nullptr;
-    }
+    if (streamk && p.partials && grid > 148) grid = 148;      // slots for 148 CTAs; without them there may be no `accum` to add into
     return launch_pdl(gemm_tc_small_kernel<FMT, BM>, dim3(grid), dim3(THREADS), C::SMEM_BYTES, st, tmap, q);
 }
 
