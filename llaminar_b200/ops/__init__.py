@@ -290,9 +290,8 @@ def attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, h
     if tensor_core is None:
         tensor_core = head_dim == 128 and max_q_len >= ATTN_TC_MIN_ROWS and _attn_tc_default()
     status = scratch.status if (tensor_core and scratch is not None) else None
-    ext().attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, head_dim, scale, max_q_len, bool(tensor_core), status,
-                       max_kv_len, scratch.part_o if status is not None else None, scratch.part_ml if status is not None else None)
-    _count()
+    _count(ext().attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, head_dim, scale, max_q_len, bool(tensor_core), status,
+                              max_kv_len, scratch.part_o if status is not None else None, scratch.part_ml if status is not None else None))
 
 
 def kv_dequant_pages(kv8: torch.Tensor, block_table: torch.Tensor, n_tokens: torch.Tensor, n_kv_heads: int, head_dim: int,

@@ -369,7 +369,8 @@ static void attn_decode(const Tensor& q, const Tensor& kv, Tensor out, const Ten
     LLM_CUDA_CHECK(llm::launch_attn_decode(p, batch, (int)n_splits, cur_stream()));
 }
 
-static void attn_prefill(const Tensor& q, const Tensor& kv, Tensor out, const Tensor& block_table, const Tensor& cu_q,
+// returns the number of launches
+static int64_t attn_prefill(const Tensor& q, const Tensor& kv, Tensor out, const Tensor& block_table, const Tensor& cu_q,
                          const Tensor& ctx_lens, int64_t n_heads, int64_t n_kv_heads, int64_t head_dim, double scale, int64_t max_q_len,
                          bool tensor_core, const OptTensor& status, int64_t max_kv_len, const OptTensor& part_o, const OptTensor& part_ml) {
     check_cuda(q, "q");
@@ -392,6 +393,7 @@ static void attn_prefill(const Tensor& q, const Tensor& kv, Tensor out, const Te
     } else {
         LLM_CUDA_CHECK(llm::launch_attn_prefill(p, (int)ctx_lens.numel(), (int)max_q_len, cur_stream()));
     }
+    return p.splits > 1 ? 2 : 1;
 }
 
 

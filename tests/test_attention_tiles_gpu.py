@@ -78,7 +78,9 @@ def test_keys_shared_out(heads, kv_heads, lens, ctx):
     sc, outs = ops.scratch_for(DEV), []
     for longest in (0, max(n + m for n, m in zip(lens, ctx))):
         outs.append(torch.full_like(q, float("nan")))
+        before = ops.launch_count()
         ops.attn_prefill(q, kv, outs[-1], table, cu, c, heads, kv_heads, 128, 1 / math.sqrt(128), max(lens), scratch=sc, max_kv_len=longest)
+        assert ops.launch_count() - before == (2 if longest >= 1024 else 1)      # a split has four tiles of 128 keys at least
         _check(outs[-1], q, cu, c, keys, values)
     assert int(sc.status[0]) == 0
 
