@@ -127,8 +127,13 @@ LLM_DEVICE void q8_unit_to_f16(const uint4& w, __half2 sc2, __half2 off2, uint32
     }
 }
 
-template <int D, bool Q8, bool CAP>                // CAP: scores are soft-capped
-__global__ void __launch_bounds__(128) paged_attn_decode_kernel(const AttnDecodeParams p) {
+// CAP: scores are soft-capped.  CTAS: CTAs of an SM that the registers have to allow (0: whatever comes out).
+// The 8-bit form at D = 128 comes out with 201 registers, two CTAs an SM; with three (168 registers) a CTA by itself is slower (256 CTAs,
+// 64 / 8 heads, 32 sequences of 700 tokens: 23 us with two, 29 with three), but many more CTAs than two an SM need them (384 CTAs,
+// 16 / 16 heads, 8 sequences of 3000 tokens in 3 splits: 55 us with two, 41 with three; 312 CTAs, 32 / 8 heads, 3 sequences of 3000: 15.1
+// and 16.9, of 8000: 29.5 and 28.8).
+template <int D, bool Q8, bool CAP, int CTAS>
+__global__ void __launch_bounds__(128, CTAS) paged_attn_decode_kernel(const AttnDecodeParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     pdl_trigger();
     pdl_wait();
@@ -468,11 +473,13 @@ cudaError_t launch_attn_decode(const AttnDecodeParams& p, int batch, int n_split
     constexpr int SLACK = 1024;
     if (p.kv_q8 && p.softcap > 0.f) return cudaErrorInvalidValue;
     auto pick = [&](auto q8, auto plain, auto capped, int smem_q8, int smem) { return p.kv_q8 ? go(q8, smem_q8 + SLACK) : go(p.softcap > 0.f ? capped : plain, smem + SLACK); };
+    const bool three = (long long)grid.x * grid.y * grid.z > 2 * sm_count() + sm_count() / 4;
     if (p.head_dim == 128)
-        return pick(paged_attn_decode_kernel<128, true, false>, paged_attn_decode_kernel<128, false, false>, paged_attn_decode_kernel<128, false, true>,
+        return pick(three ? paged_attn_decode_kernel<128, true, false, 3> : paged_attn_decode_kernel<128, true, false, 0>,
+                    paged_attn_decode_kernel<128, false, false, 0>, paged_attn_decode_kernel<128, false, true, 0>,
                     DecodeSmem<128, true>::BYTES, DecodeSmem<128, false>::BYTES);
     if (p.head_dim == 64)
-        return pick(paged_attn_decode_kernel<64, true, false>, paged_attn_decode_kernel<64, false, false>, paged_attn_decode_kernel<64, false, true>,
+        return pick(paged_attn_decode_kernel<64, true, false, 0>, paged_attn_decode_kernel<64, false, false, 0>, paged_attn_decode_kernel<64, false, true, 0>,
                     DecodeSmem<64, true>::BYTES, DecodeSmem<64, false>::BYTES);
     return cudaErrorInvalidValue;
 }
