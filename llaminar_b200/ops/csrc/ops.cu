@@ -207,7 +207,9 @@ cudaError_t launch_mtp_concat_norm(const float* emb, const float* hidden, const 
 // has the loads of eight heads in flight (108 us; 2048 tokens, 32 / 8 heads: 18.2 instead of 27.2).  Short chunks and decode steps keep a warp per head: there the number of warps in
 // flight is what counts.
 // ------------------------------------------------------------------------------------------------
-template <int D, int HEADS>
+// WORDS: a lane's two values of a half are one word (D = 128, rows that start on words).  Decided on the host: both ways in one kernel made
+// the form of a head per warp 3 to 7 % slower (600 tokens, 32 / 8 heads, 8-bit cache: 10.4 us, 9.7 so).
+template <int D, int HEADS, bool WORDS>
 __global__ void __launch_bounds__(128) rope_kv_kernel(const RopeKVParams p) {
     constexpr int EPL = D / 64;                          // elements per lane in each half
     pdl_trigger();
@@ -219,15 +221,13 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const RopeKVParams p) {
     const int t = item / parts, h0 = item % parts * HEADS;
     const __nv_bfloat16* src = p.qkv + ((size_t)t * heads_total + h0) * D;
     const int pos = p.positions[t];
-    // a lane's two values of a half as one word, where the rows start on words
-    const bool words = ((reinterpret_cast<uintptr_t>(p.qkv) | reinterpret_cast<uintptr_t>(p.q_out) | reinterpret_cast<uintptr_t>(p.kv)) & 3) == 0;
     float a[HEADS][EPL], b[HEADS][EPL];                  // first and second halves of the heads
 #pragma unroll
     for (int j = 0; j < HEADS; ++j)
 #pragma unroll
         for (int e = 0; e < EPL; ++e) {
             const bool in = HEADS == 1 || h0 + j < heads_total;
-            if (EPL == 2 && words) {
+            if constexpr (WORDS) {
                 if (e) continue;
                 const uint32_t* x = reinterpret_cast<const uint32_t*>(src + j * D) + lane;
                 const uint32_t u = in ? x[0] : 0u, v = in ? x[D / 4] : 0u;
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const RopeKVParams p) {
             }
             dst = p.kv + ((page * 2 + (is_k ? 0 : 1)) * p.n_kv_heads + kvh) * (size_t)(PAGE * D) + (size_t)(pos % PAGE) * D;
         }
-        if (EPL == 2 && words) {
+        if constexpr (WORDS) {
             uint32_t* x = reinterpret_cast<uint32_t*>(dst) + lane;
             x[0] = pack_bf16(a[j][0], a[j][EPL - 1]);
             x[D / 4] = pack_bf16(b[j][0], b[j][EPL - 1]);
@@ -345,10 +345,11 @@ cudaError_t launch_rope_kv(const RopeKVParams& p, cudaStream_t st) {
     const long long shared = (long long)p.n_tokens * ((heads + MANY - 1) / MANY);          // warps that take eight heads each
     const bool many = shared >= 148 * 32;                // two thirds of the warps that the GPU holds of this kernel
     const int grid = many ? (int)((shared + 3) / 4) : (p.n_tokens * heads + 3) / 4;
-    if (p.head_dim == 128) return launch_pdl(many ? rope_kv_kernel<128, MANY> : rope_kv_kernel<128, 1>, dim3(grid), dim3(128), 0, st, p);
-    else if (p.head_dim == 64) return launch_pdl(many ? rope_kv_kernel<64, MANY> : rope_kv_kernel<64, 1>, dim3(grid), dim3(128), 0, st, p);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    auto go = [&](auto one, auto eight) { return launch_pdl(many ? eight : one, dim3(grid), dim3(128), 0, st, p); };
+    if (p.head_dim == 64) return go(rope_kv_kernel<64, 1, false>, rope_kv_kernel<64, MANY, false>);
+    if (p.head_dim != 128) return cudaErrorInvalidValue;
+    const bool words = ((reinterpret_cast<uintptr_t>(p.qkv) | reinterpret_cast<uintptr_t>(p.q_out) | reinterpret_cast<uintptr_t>(p.kv)) & 3) == 0;
+    return words ? go(rope_kv_kernel<128, 1, true>, rope_kv_kernel<128, MANY, true>) : go(rope_kv_kernel<128, 1, false>, rope_kv_kernel<128, MANY, false>);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -9,8 +9,10 @@ DEV = "cuda"
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("heads,kv_heads", [(16, 4), (7, 1), (1, 1), (12, 2)])
 @pytest.mark.parametrize("q8", [False, True])
-def test_chunk_equals_its_tokens(D, heads, kv_heads, q8):
-    """The values of a chunk are, bit for bit, those of its tokens in portions that a warp per head takes."""
+@pytest.mark.parametrize("odd", [0, 1])
+def test_chunk_equals_its_tokens(D, heads, kv_heads, q8, odd):
+    """The values of a chunk are, bit for bit, those of its tokens in portions that a warp per head takes; rows that start between two
+    words too."""
     from llaminar_b200 import ops
     total = heads + 2 * kv_heads
     T = 4736 // ((total + 7) // 8) + 5
@@ -27,7 +29,8 @@ def test_chunk_equals_its_tokens(D, heads, kv_heads, q8):
         q = torch.zeros(T, heads, D, dtype=torch.bfloat16, device=DEV)
         for t in range(0, T, step):
             s = slice(t, min(t + step, T))
-            ops.rope_kv(qkv[s].clone(), q[s], kv, qn, kn, pos[s], sid[s], table, heads, kv_heads, D, 1e6, 1e-6)
+            rows = torch.empty(qkv[s].numel() + odd, dtype=torch.bfloat16, device=DEV)[odd if step == T else 0:][:qkv[s].numel()].view_as(qkv[s]).copy_(qkv[s])
+            ops.rope_kv(rows, q[s], kv, qn, kn, pos[s], sid[s], table, heads, kv_heads, D, 1e6, 1e-6)
         return q, kv
 
     (q, kv), (q1, kv1) = run(T), run(300)
