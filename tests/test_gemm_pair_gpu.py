@@ -35,8 +35,10 @@ def test_pair_edges(qt, m, n, k):
     bias, h0 = torch.randn(n, generator=g, device=DEV), torch.randn(m, n, generator=g, device=DEV)
     h = h0.clone()
     ops.gemm(pw, x, h, epi=ops.EPI_RESID, bias=bias, scratch=sc)
-    whole = torch.empty(m, n, dtype=torch.float32, device=DEV)
+    whole, bare, added = torch.empty(m, n, dtype=torch.float32, device=DEV), torch.empty(m, n, dtype=torch.float32, device=DEV), h0.clone()
     ops.gemm(pw, x, whole, bias=bias, scratch=sc)
+    ops.gemm(pw, x, bare, scratch=sc)
+    ops.gemm(pw, x, added, epi=ops.EPI_RESID, scratch=sc)
     gu = n // 32 * 16
     row = raw.numel() // n
     raw2, _, n2, _ = interleave_gate_up(raw[:row * gu], raw[row * gu:row * 2 * gu], qt, gu, k)
@@ -45,6 +47,7 @@ def test_pair_edges(qt, m, n, k):
     torch.cuda.synchronize()
     assert int(sc.status[0]) == 0
     assert _rel(out, ref) < REL and _rel(h - h0 - bias, ref) < REL and _rel(whole - bias, ref) < REL
+    assert torch.equal(added, h0 + bare)                 # the same sums, and one rounded addition
     assert bool((wide[m:] == 7.0).all()) and bool((wide[:, n:] == 7.0).all())
     assert _rel(act, torch.nn.functional.silu(ref[:, :gu]) * ref[:, gu:2 * gu]) < 2 * REL
 
