@@ -614,6 +614,21 @@ static cudaError_t launch_fmt(const GemmTcParams& p, int bm, int ks, cudaStream_
     return cudaErrorInvalidValue;
 }
 
+// Few rows of a narrow and long matrix leave most pairs without a tile; there the kernel here, which splits K, can be the faster one
+// (its partial sums meet by atomics, in the order they arrive).  Both times in us, as 17 matrices of 512 x 2048 to 5120 x 25600 in four
+// formats showed them at 129 to 512 rows (the rule loses more than 5 % in 7 of 560 calls and 13 % at most):
+//   pairs: 2, and the chunks of the busiest pair at the conversion's rate; the residual's epilogue 4 more
+//   split: 22, 1.2 for every chunk of the busiest CTA, 36 for every million outputs (atomics, and the last CTA's epilogue)
+// Examples (pairs, split): 4096 x 12288 Q4_K + residual, 129 rows 71, 53; 256 rows 73, 73; 2560 x 9728 Q8_0, 129 rows 73, 45; 4096 x 4096
+// Q4_K, 129 rows 24, 46.
+static bool splits_k(const GemmTcParams& p, int ks) {
+    const double rate = p.fmt == FMT_Q4_K || p.fmt == FMT_Q4_0 ? 1.35 : p.fmt == FMT_Q6_K ? 1.57 : p.fmt == FMT_Q5_K ? 1.67 : 1.84;
+    const int kb = p.k / 256, n_tiles = (p.n + 127) / 128, m_tiles = (p.m + 255) / 256;
+    const int pairs = (n_tiles + 1) / 2 * m_tiles, ctas = n_tiles * m_tiles * ks;
+    const double by_pairs = 2 + (pairs + 73) / 74 * kb * rate + (p.epi == EPI_RESID ? 4 : 0);
+    return 22 + (ctas + 147) / 148 * ((kb + ks - 1) / ks) * 1.2 + 36e-6 * p.n * p.m < by_pairs;
+}
+
 cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st) {
     if (p.m <= 0) return cudaSuccess;
     const void* xa = p.ag_on ? static_cast<const void*>(p.ag.stage) : static_cast<const void*>(p.x);
@@ -652,10 +667,7 @@ cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st) {
     // Q4_K scales that the short conversion does not take, and more groups than the pairs keep offsets for.
     if (!p.rs_on && !p.ag_on && !p.debug && p.groups <= 256 && !wide) {
         if (p.groups > 0) return launch_gemm_tc_pair(p, bm, st);
-        // (up to 256 rows of a narrow and long matrix leave most pairs without a tile: there this kernel splits K instead.
-        // 5120 x 25600 Q4_K, 160 rows: 99 us here, 124 us there; 4096 x 12288: 62 and 63 us.)
-        const bool narrow = ks > 1 && p.k >= 64 * 256 && (p.n + 127) / 128 * ((p.m + 255) / 256) <= 74;
-        if (bm == 256 && p.ksplit <= 1 && !narrow) return launch_gemm_tc_pair(p, gemm_pair_tokens(p.fmt, p.m, p.n, p.k), st);
+        if (bm == 256 && p.ksplit <= 1 && !(ks > 1 && splits_k(p, ks))) return launch_gemm_tc_pair(p, gemm_pair_tokens(p.fmt, p.m, p.n, p.k), st);
     }
     switch (p.fmt) {
         case FMT_Q4_K: return launch_fmt<FMT_Q4_K>(p, bm, ks, st);

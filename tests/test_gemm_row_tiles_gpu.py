@@ -50,3 +50,24 @@ def test_row_tile_edges(qt, m, n, k):
     assert bool((wide[m:] == 7.0).all()) and bool((wide[:, n:] == 7.0).all())
     gate, up = ref[:, :gu], ref[:, gu:2 * gu]
     assert _rel(act, torch.nn.functional.silu(gate) * up) < 2.4e-2
+
+
+@pytest.mark.parametrize("qt", [GGMLType.Q4_K, GGMLType.Q8_0])
+@pytest.mark.parametrize("n,k", [(640, 16384), (2000, 9728), (300, 4096)])
+@pytest.mark.parametrize("m", [129, 160, 256, 300])
+def test_long_and_narrow(qt, n, k, m):
+    """Shapes around the line where K is split between CTAs whose sums meet by atomics: values, and counters and sums back at zero."""
+    from llaminar_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(m)
+    raw = quantize(torch.randn(n, k, generator=g, device=DEV) * 0.05, qt)
+    pw, sc = ops.pack_matrix(raw, qt, n, k), ops.scratch_for(DEV)
+    sc.status.zero_()
+    x = torch.randn(m, k, generator=g, device=DEV).to(torch.bfloat16)
+    ref = x.float() @ dequantize(raw, qt, (n, k)).T
+    out, h0 = torch.empty(m, n, dtype=torch.bfloat16, device=DEV), torch.randn(m, n, generator=g, device=DEV)
+    h = h0.clone()
+    ops.gemm(pw, x, out, scratch=sc)
+    ops.gemm(pw, x, h, epi=ops.EPI_RESID, scratch=sc)
+    torch.cuda.synchronize()
+    assert int(sc.status[0]) == 0 and int(sc.tickets.abs().sum()) == 0 and float(sc.accum.abs().max()) == 0
+    assert _rel(out, ref) < 1.2e-2 and _rel(h - h0, ref) < 1.2e-2
