@@ -99,7 +99,8 @@ struct Tiles {
     }
 };
 
-template <int FMT>
+// RESID: the residual epilogue, else store or SwiGLU (one kernel with all of them was 2 to 5 % slower from Q6_K)
+template <int FMT, bool RESID>
 __global__ void __launch_bounds__(THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmTcParams p, const int bt) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_full[SLOTS], s_empty[SLOTS], s_acc_full, s_acc_empty;
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_pair_kernel(const __grid_cons
             for (int b = 0; b < 4; ++b) {
                 const int c0 = (set + 2 * b) * 32, m0 = t.row0 + c0;
                 if (c0 >= t.cols) break;
-                if (p.epi == EPI_SWIGLU) {
+                if (!RESID && p.epi == EPI_SWIGLU) {
                     // rows of a 32-row group: 16 gate rows, then the 16 matching up rows.  Lanes l and l + 16 hold one output column;
                     // the lower lane finishes the even tokens and the upper lane the odd ones, so one exchange serves two.
                     const int col = tile_n * 64 + g * 16 + (lane & 15);
@@ -187,26 +188,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_pair_kernel(const __grid_cons
                 }
                 if (n_row >= p.n) continue;
                 const float bias = p.bias ? p.bias[n_row] : 0.f;
-                if (p.epi == EPI_RESID) {
+                if constexpr (RESID) {
+                    // one addition to every element, made in L2: read, added and written here they were a chain of sixteen trips
+                    // to L2 (4096 x 4096 Q4_K, 1024 rows: 42 us, 34 so; 4096 rows: 172 and 128)
                     float* h = static_cast<float*>(p.out) + (size_t)m0 * p.out_stride + n_row;
-                    if (!p.bias) {
-                        // one addition to every element, made in L2: read, added and written here they were a chain of sixteen trips
-                        // to L2 (4096 x 4096 Q4_K, 1024 rows: 42 us, 34 so; 4096 rows: 172 and 128)
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (m0 + j < t.row_hi)
-                                asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(h + (size_t)j * p.out_stride), "f"(__uint_as_float(r[b][j])) : "memory");
-                        continue;
-                    }
-#pragma unroll
-                    for (int j0 = 0; j0 < 32; j0 += 8) {
-                        float old[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) old[j] = m0 + j0 + j < t.row_hi ? h[(size_t)(j0 + j) * p.out_stride] : 0.f;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (m0 + j0 + j < t.row_hi) h[(size_t)(j0 + j) * p.out_stride] = old[j] + __uint_as_float(r[b][j0 + j]) + bias;
-                    }
+                    for (int j = 0; j < 32; ++j)
+                        if (m0 + j < t.row_hi)
+                            asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(h + (size_t)j * p.out_stride), "f"(__uint_as_float(r[b][j]) + bias) : "memory");
                     continue;
                 }
 #pragma unroll
@@ -338,11 +327,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_pair_kernel(const __grid_cons
     if (warp == DEQUANT_WARPS + 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-template <int FMT>
+template <int FMT, bool RESID>
 static cudaError_t launch_one(const GemmTcParams& p, int bt, cudaStream_t st) {
     static bool attr_set = false;
     if (!attr_set) {
-        const cudaError_t e = raise_smem(gemm_pair_kernel<FMT>, SMEM_BYTES);
+        const cudaError_t e = raise_smem(gemm_pair_kernel<FMT, RESID>, SMEM_BYTES);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
@@ -358,7 +347,11 @@ static cudaError_t launch_one(const GemmTcParams& p, int bt, cudaStream_t st) {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<FMT>, map, p, bt);
+    return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<FMT, RESID>, map, p, bt);
+}
+template <int FMT>
+static cudaError_t launch_fmt(const GemmTcParams& p, int bt, cudaStream_t st) {
+    return p.epi == EPI_RESID ? launch_one<FMT, true>(p, bt, st) : launch_one<FMT, false>(p, bt, st);
 }
 
 }  // namespace tcp
@@ -382,12 +375,12 @@ int gemm_pair_tokens(int fmt, int m, int n, int k) {
 cudaError_t launch_gemm_tc_pair(const GemmTcParams& p, int bt, cudaStream_t st) {
     if (bt < 32 || bt > 256 || bt % 32 || p.groups > tcp::MAX_GROUPS) return cudaErrorInvalidValue;
     switch (p.fmt) {
-        case FMT_Q4_K: return tcp::launch_one<FMT_Q4_K>(p, bt, st);
-        case FMT_Q5_K: return tcp::launch_one<FMT_Q5_K>(p, bt, st);
-        case FMT_Q6_K: return tcp::launch_one<FMT_Q6_K>(p, bt, st);
-        case FMT_Q8_0: return tcp::launch_one<FMT_Q8_0>(p, bt, st);
-        case FMT_Q4_0: return tcp::launch_one<FMT_Q4_0>(p, bt, st);
-        case FMT_IQ3_S: return tcp::launch_one<FMT_IQ3_S>(p, bt, st);
+        case FMT_Q4_K: return tcp::launch_fmt<FMT_Q4_K>(p, bt, st);
+        case FMT_Q5_K: return tcp::launch_fmt<FMT_Q5_K>(p, bt, st);
+        case FMT_Q6_K: return tcp::launch_fmt<FMT_Q6_K>(p, bt, st);
+        case FMT_Q8_0: return tcp::launch_fmt<FMT_Q8_0>(p, bt, st);
+        case FMT_Q4_0: return tcp::launch_fmt<FMT_Q4_0>(p, bt, st);
+        case FMT_IQ3_S: return tcp::launch_fmt<FMT_IQ3_S>(p, bt, st);
     }
     return cudaErrorInvalidValue;
 }
