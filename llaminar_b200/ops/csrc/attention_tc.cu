@@ -96,7 +96,7 @@ LLM_DEVICE void finish_row(const AttnPrefillParams& p, size_t at, int head, floa
 enum Bar { K_FULL = 0, K_EMPTY = 2, V_FULL = 4, V_EMPTY = 6, Q_FULL = 8, S_FULL = 9, P_FULL = 11, O_FULL = 13, N_BARS = 15 };
 
 template <bool CAP>                                // scores are soft-capped
-__global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPrefillParams p, int* status) {
+__global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const AttnPrefillTcParams p, int* status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t s_bars[N_BARS];
     __shared__ uint32_t s_tmem;
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
 }
 
 // The splits' results of a query row, a warp per row and head: rescaled to the largest maximum, summed up in split order.
-__global__ void __launch_bounds__(128) paged_attn_prefill_merge_kernel(const AttnPrefillParams p, int pairs) {
+__global__ void __launch_bounds__(128) paged_attn_prefill_merge_kernel(const AttnPrefillTcParams p, int pairs) {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31, G = p.n_heads / p.n_kv_heads, head = blockIdx.y, kvh = head / G, seq = blockIdx.z;
@@ -443,7 +443,7 @@ int attn_prefill_tc_splits(int n_heads, int n_kv_heads, int n_seqs, int max_q_le
     return s < 2 ? 1 : (int)s;
 }
 
-cudaError_t launch_attn_prefill_tc(const AttnPrefillParams& p, int n_seqs, int max_q_len, int* status, cudaStream_t st) {
+cudaError_t launch_attn_prefill_tc(const AttnPrefillTcParams& p, int n_seqs, int max_q_len, int* status, cudaStream_t st) {
     if (n_seqs == 0 || max_q_len == 0) return cudaSuccess;
     if (p.head_dim != atc::D || p.n_heads % p.n_kv_heads) return cudaErrorInvalidValue;
     // the cache as a matrix of head_dim columns: 64 rows per page, K or V, and head

@@ -375,7 +375,7 @@ static int64_t attn_prefill(const Tensor& q, const Tensor& kv, Tensor out, const
                          bool tensor_core, const OptTensor& status, int64_t max_kv_len, const OptTensor& part_o, const OptTensor& part_ml) {
     check_cuda(q, "q");
     const c10::cuda::CUDAGuard guard(q.device());
-    llm::AttnPrefillParams p{};
+    llm::AttnPrefillTcParams p{};
     p.q = static_cast<const __nv_bfloat16*>(q.data_ptr()); p.kv = static_cast<const __nv_bfloat16*>(kv.data_ptr());
     p.out = static_cast<__nv_bfloat16*>(out.data_ptr());
     p.block_table = static_cast<const int*>(block_table.data_ptr()); p.cu_q = static_cast<const int*>(cu_q.data_ptr());

@@ -168,7 +168,7 @@ void attn_prefill(const Tensor& q, const Tensor& kv, const Tensor& out, const Te
     TORCH_CHECK(block_table.size(0) >= n && cu_q.numel() == n + 1, "sequences");
     const bool gate_heads = gate_rows(gate, T, H, D);
     if (n == 0 || max_q_len == 0) return;
-    llm::AttnPrefillParams p = {};
+    llm::AttnPrefillTcParams p = {};
     p.q = bf16(q, "q"); p.kv = bf16(kv, "kv"); p.out = const_cast<__nv_bfloat16*>(bf16(out, "out"));
     p.block_table = ints(block_table, "block_table"); p.cu_q = ints(cu_q, "cu_q"); p.ctx_lens = ints(ctx_lens, "ctx_lens");
     p.n_heads = H; p.n_kv_heads = kv.size(2); p.head_dim = D; p.max_pages = block_table.size(1); p.scale = scale; p.n_pages = kv.size(0);

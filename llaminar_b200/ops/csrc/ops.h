@@ -47,7 +47,10 @@ struct AttnPrefillParams {
     size_t gate_row;               // even
     int gate_heads, chunk;
     float softcap;
-    // tcgen05 kernel: the keys of a query tile are shared out between `splits` CTAs, whose results meet in a second launch
+};
+// tcgen05 kernel: the keys of a query tile are shared out between `splits` CTAs, whose results meet in a second launch.  (A struct of its
+// own: three more parameters made the mma.sync kernel come out up to 18 % slower, 32 sequences of 16 tokens, 16 / 16 heads 18.5 -> 21.7 us.)
+struct AttnPrefillTcParams : AttnPrefillParams {
     int splits;                    // 0 or 1: not split
     float* part_o;                 // [2 * pairs of query tiles][splits][128][head_dim], pairs counted over the grid
     float* part_ml;                // [2 * pairs][splits][128][2] maxima and sums
@@ -57,7 +60,7 @@ int attn_decode_pick_splits(int batch, int n_kv_heads, int max_pages_in_use);
 cudaError_t launch_attn_decode(const AttnDecodeParams& p, int batch, int n_splits, cudaStream_t st);
 cudaError_t launch_attn_prefill(const AttnPrefillParams& p, int n_seqs, int max_q_len, cudaStream_t st);
 // tcgen05 version (head_dim 128 only); `status` (optional) receives STATUS_TIMEOUT if a pipeline wait gave up
-cudaError_t launch_attn_prefill_tc(const AttnPrefillParams& p, int n_seqs, int max_q_len, int* status, cudaStream_t st);
+cudaError_t launch_attn_prefill_tc(const AttnPrefillTcParams& p, int n_seqs, int max_q_len, int* status, cudaStream_t st);
 // splits that a call of these sizes should have, within a scratch of that many floats (part_o, part_ml)
 int attn_prefill_tc_splits(int n_heads, int n_kv_heads, int n_seqs, int max_q_len, int max_kv_len, long long part_o, long long part_ml);
 
