@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
             }
             ok = ok && mbar_wait_warp(bar(O_FULL + slot), 0, abort_flag);
             const float sum_l = l;
-            float odd = 0.f;                                       // NaN once a value of the row's O is not finite
+            float odd[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};       // NaN once a value of the row's O is not finite
             if (ok && splits > 1) {
                 tc_fence_after();
                 const size_t at = part + (size_t)slot * splits * BQ + row;
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
                     uint32_t r[32];
                     tmem_ld_n<32>(t_o + c * 32, r);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) odd = fmaf(__uint_as_float(r[i]), 0.f, odd);
+                    for (int i = 0; i < 32; ++i) odd[i & 7] = fmaf(__uint_as_float(r[i]), 0.f, odd[i & 7]);
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
                         dst[c * 8 + u] = make_float4(__uint_as_float(r[4 * u]), __uint_as_float(r[4 * u + 1]), __uint_as_float(r[4 * u + 2]), __uint_as_float(r[4 * u + 3]));
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
                     uint32_t r[32];
                     tmem_ld_n<32>(t_o + c * 32, r);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) odd = fmaf(__uint_as_float(r[i]), 0.f, odd);
+                    for (int i = 0; i < 32; ++i) odd[i & 7] = fmaf(__uint_as_float(r[i]), 0.f, odd[i & 7]);
                     if (row < rows) {
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(THREADS, 1) paged_attn_prefill_tc_kernel(const
             // A masked key has P = 0, and 0 times an infinity or NaN in its V row (a later token, or what the page held before) is
             // NaN.  Rows that are not finite although their scores are, and that have such a key in their tiles, are computed again
             // over their own keys alone.
-            unsigned again = __ballot_sync(0xffffffffu, ok && row < rows && odd != 0.f && fabsf(sum_l) <= 3.4e38f);
+            const float any = ((odd[0] + odd[1]) + (odd[2] + odd[3])) + ((odd[4] + odd[5]) + (odd[6] + odd[7]));
+            unsigned again = __ballot_sync(0xffffffffu, ok && row < rows && any != 0.f && fabsf(sum_l) <= 3.4e38f);
             if (again) __syncwarp();                               // the stores above come before the ones below
 #pragma unroll 1
             for (; again; again &= again - 1) {
