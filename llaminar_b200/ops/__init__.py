@@ -280,15 +280,31 @@ def attn_decode(q, kv, out, block_table, seq_lens, n_heads, n_kv_heads, head_dim
     _count()
 
 
+def _few_keys_many_ctas(n_seqs: int, n_heads: int, n_kv_heads: int, max_q_len: int, max_kv_len: int) -> bool:
+    """Many short prompts: whether the mma.sync kernel is the faster one.  A CTA of the tcgen05 kernel (two slots of 128 query rows) has an
+    SM to itself and costs about 8.5 us (7.5 with one slot), 2 more per further tile of 128 keys; of the other's (64 query rows) three
+    share an SM for 8 to 9 us, 4.5 more per further page.  Measured, 16 / 16 heads, 32 sequences of 16 tokens: 29 and 18.5 us; 32 / 8
+    heads, 32 of 16: 35 and 27; 16 / 16 heads, 128 of 5 behind 128: 132 and 91; of 1380 calls of more than one CTA an SM the rule loses
+    more than 5 % in two.  Up to one CTA an SM the two are within a microsecond, and the tcgen05 kernel overlaps its predecessor's end."""
+    if max_kv_len <= 0 or max_q_len <= 0 or n_kv_heads <= 0 or n_heads % n_kv_heads:
+        return False
+    G, sms = n_heads // n_kv_heads, 148
+    pairs = (-(-max_q_len // 128) * G + 1) // 2
+    ctas, others = pairs * n_kv_heads * n_seqs, -(-max_q_len // 64) * n_heads * n_seqs
+    tc = -(-ctas // sms) * ((7.5 if G == 1 and max_q_len <= 128 else 8.5) + 2 * (-(-max_kv_len // 128) - 1))
+    return ctas > sms and -(-others // (3 * sms)) * (8 + min(max_q_len, 64) / 64 + 4.5 * (-(-max_kv_len // 64) - 1)) < tc
+
+
 def attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, head_dim, scale, max_q_len,
                  tensor_core: bool | None = None, scratch: "Scratch | None" = None, max_kv_len: int = 0) -> None:
     """Causal GQA attention of a prefill chunk over the paged cache.  ``tensor_core`` picks the tcgen05 kernel (head_dim 128),
-    otherwise the mma.sync kernel runs.  Default: the tcgen05 kernel wherever it fits; it is the faster one from ATTN_TC_MIN_ROWS
-    query rows on (32 / 8 heads: 8.9 vs 11.3 us at 16 rows, 23.6 vs 82.6 at 1024, 164 vs 785 at 4096, 120 vs 414 at 500 rows
-    behind 7000 tokens); LLAMINAR_ATTN_TC=0 turns it off.  With ``max_kv_len`` (the longest context and chunk of the batch; 0:
+    otherwise the mma.sync kernel runs.  Default: the tcgen05 kernel wherever it fits, from ATTN_TC_MIN_ROWS query rows on (32 / 8
+    heads: 8.9 vs 11.3 us at 16 rows, 23.6 vs 82.6 at 1024, 164 vs 785 at 4096, 120 vs 414 at 500 rows behind 7000 tokens), but for
+    many short prompts (`_few_keys_many_ctas`); LLAMINAR_ATTN_TC=0 turns it off.  With ``max_kv_len`` (the longest context and chunk of the batch; 0:
     unknown) and ``scratch`` it shares the keys of few query rows out between CTAs."""
     if tensor_core is None:
-        tensor_core = head_dim == 128 and max_q_len >= ATTN_TC_MIN_ROWS and _attn_tc_default()
+        tensor_core = (head_dim == 128 and max_q_len >= ATTN_TC_MIN_ROWS and _attn_tc_default()
+                       and not _few_keys_many_ctas(ctx_lens.numel(), n_heads, n_kv_heads, max_q_len, max_kv_len))
     status = scratch.status if (tensor_core and scratch is not None) else None
     _count(ext().attn_prefill(q, kv, out, block_table, cu_q, ctx_lens, n_heads, n_kv_heads, head_dim, scale, max_q_len, bool(tensor_core), status,
                               max_kv_len, scratch.part_o if status is not None else None, scratch.part_ml if status is not None else None))

@@ -85,6 +85,18 @@ def test_keys_shared_out(heads, kv_heads, lens, ctx):
     assert int(sc.status[0]) == 0
 
 
+def test_many_short_prompts():
+    """More CTAs than SMs and few keys each: the other kernel, by the sizes alone."""
+    from llaminar_b200 import ops
+    lens = [1 + i % 10 for i in range(40)]
+    ctx = [i % 7 for i in range(40)]
+    q, kv, table, cu, c, keys, values = _case(16, 16, lens, ctx, False, 4)
+    out, sc = torch.full_like(q, float("nan")), ops.scratch_for(DEV)
+    assert ops._few_keys_many_ctas(40, 16, 16, 10, 16)
+    ops.attn_prefill(q, kv, out, table, cu, c, 16, 16, 128, 1 / math.sqrt(128), max(lens), scratch=sc, max_kv_len=16)
+    _check(out, q, cu, c, keys, values)
+
+
 @pytest.mark.parametrize("window,softcap,sink", [(1, 0.0, False), (100, 0.0, True), (129, 20.0, False), (0, 30.0, True)])
 def test_masks(window, softcap, sink):
     from llaminar_b200.ops import grouped
