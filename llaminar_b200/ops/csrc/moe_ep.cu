@@ -374,8 +374,9 @@ cudaError_t launch_moe_route(const MoeRouteParams& p, cudaStream_t st) {
         (p.items != nullptr && p.tokens * p.top_k > ROUTE_MAX_PAIRS))
         return cudaErrorInvalidValue;
     constexpr int MANY = 8;
-    // at least three CTAs for every SM and a row of d floats per token that fits
-    const bool many = p.items == nullptr && p.tokens >= 148 * 3 && (size_t)MANY * (p.d + ROUTE_MAX_EXPERTS) * sizeof(float) <= 100 * 1024;
+    // (and rows of d floats that fit).  Up to 444 tokens, three CTAs an SM, a CTA per token is one wave and as fast or faster: 128 experts of
+    // 2048, 444 tokens 28 us, 32 with eight tokens; 500 tokens 34 and 32, 888 50 and 32
+    const bool many = p.items == nullptr && p.tokens > 148 * 3 && (size_t)MANY * (p.d + ROUTE_MAX_EXPERTS) * sizeof(float) <= 100 * 1024;
     const int tok = many ? MANY : 1;
     const size_t dyn = max((size_t)tok * (p.d + ROUTE_MAX_EXPERTS) * sizeof(float), p.items ? (size_t)p.tokens * p.top_k * sizeof(int) : (size_t)0);
     auto kernel = many ? moe_route_kernel<MANY> : moe_route_kernel<1>;
