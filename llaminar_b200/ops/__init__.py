@@ -10,6 +10,7 @@ from dataclasses import dataclass
 
 import torch
 
+from ..gguf.constants import GGMLType
 from . import build as _build
 from .layout import FMT_IDS, PackedWeight, can_pack, pack_experts, pack_matrix  # noqa: F401
 
@@ -169,8 +170,20 @@ def gemm_grouped(pw: PackedWeight, x: torch.Tensor, out: torch.Tensor, row_off: 
     _count()
 
 
-def _stream_args(sc: Scratch | None):
-    return (sc.partials, sc.tickets, sc.status) if sc is not None else (None, None, None)
+def _streams(pw: PackedWeight, pairs: int, z_max: int) -> bool:
+    """Whether `pairs` (token, slot) pairs run on the streaming kernel.  From Q6_K the register-path kernel is the faster one where its CTAs,
+    at the items to be expected, fill most of one wave of two an SM and no more (us streaming and there; 128 experts of 768 x 2048, 2
+    tokens, down 17.4 and 12.8; 3 tokens, gate | up 24.1 and 20.2; 4 tokens, down 20.6 and 23.2).  Of 120 measured calls 25 are more
+    than 4 % off if all stream, 11 with this.  Other formats stream."""
+    if pw.qtype != GGMLType.Q6_K or pw.n_experts < 1:
+        return True
+    used = pw.n_experts * (1 - (1 - 1 / pw.n_experts) ** pairs)          # experts that so many pairs meet
+    split = min(max(1, 592 // (pw.n_tiles * z_max)), max(1, pw.k_blocks // 2))      # the register path's split of K
+    return not 150 <= (used + max(0.0, pairs / 4 - used / 2)) * pw.n_tiles * split <= 290
+
+
+def _stream_args(sc: Scratch | None, stream: bool = True):
+    return (sc.partials, sc.tickets, sc.status) if sc is not None and stream else (None, None, None)
 
 
 def moe_gate_up(pw: PackedWeight, h, norm_w, eps, act, items, n_items, top_k, z_max, scratch: Scratch | None = None) -> None:
@@ -180,7 +193,7 @@ def moe_gate_up(pw: PackedWeight, h, norm_w, eps, act, items, n_items, top_k, z_
         accum, tickets = None, None
     stride = pw.n_tiles * pw.k_blocks * pw.chunk_bytes
     _count(ext().moe_gemv(pw.data, pw.fmt, pw.n, pw.k, stride, h, norm_w, eps, act, EPI_SWIGLU, items, n_items, top_k, z_max,
-                          accum, tickets, None, None, top_k, 0, 0, None, None, None, *_stream_args(scratch)))
+                          accum, tickets, None, None, top_k, 0, 0, None, None, None, *_stream_args(scratch, _streams(pw, h.shape[0] * top_k, z_max))))
 
 
 def moe_down_combine(pw: PackedWeight, act, yslot, items, n_items, z_max, ids, wts, top_k, e0, n_local, h, tile_tickets,
@@ -192,7 +205,7 @@ def moe_down_combine(pw: PackedWeight, act, yslot, items, n_items, z_max, ids, w
         accum, tickets = None, None
     stride = pw.n_tiles * pw.k_blocks * pw.chunk_bytes
     _count(ext().moe_gemv(pw.data, pw.fmt, pw.n, pw.k, stride, act, None, 0.0, yslot, EPI_MOE_COMBINE, items, n_items, 1, z_max,
-                          accum, tickets, ids, wts, top_k, e0, n_local, h, tile_tickets, tp, *_stream_args(scratch)))
+                          accum, tickets, ids, wts, top_k, e0, n_local, h, tile_tickets, tp, *_stream_args(scratch, _streams(pw, ids.numel(), z_max))))
 
 
 def gemm(pw: PackedWeight, x: torch.Tensor, out: torch.Tensor, *, epi: int = EPI_STORE, bias: torch.Tensor | None = None,

@@ -22,3 +22,20 @@ def test_many_short_prompts_take_the_kernel_of_small_ctas():
     for case in ((1, 32, 8, 5, 5), (8, 32, 8, 10, 10), (64, 16, 16, 10, 1010), (1, 32, 8, 4096, 4096), (8, 64, 8, 1020, 1020),
                  (32, 32, 8, 200, 200), (64, 16, 16, 10, 0), (1, 7, 2, 5, 5)):
         assert not few(*case), case
+
+
+def test_few_rows_of_6_bit_experts_keep_the_register_path():
+    import torch
+
+    from llaminar_b200.gguf import GGMLType
+    from llaminar_b200.ops import _streams
+    from llaminar_b200.ops.layout import FMT_IDS, PackedWeight
+
+    def stack(qt, E, n, k):
+        return PackedWeight(FMT_IDS[qt], qt, n, k, n // 128, k // 256, torch.empty(0), E)
+
+    z = lambda E, pairs: E + (pairs + 3) // 4
+    for E, n, k, pairs, streams in ((128, 2048, 768, 16, False), (128, 1536, 2048, 24, False), (128, 2048, 768, 32, True), (128, 1536, 2048, 8, True),
+                                    (8, 4096, 1024, 8, False), (8, 4096, 1024, 64, True)):
+        assert _streams(stack(GGMLType.Q6_K, E, n, k), pairs, z(E, pairs)) == streams, (E, n, k, pairs)
+        assert _streams(stack(GGMLType.Q4_K, E, n, k), pairs, z(E, pairs))
