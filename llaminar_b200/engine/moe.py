@@ -9,8 +9,9 @@ expert.  Under expert parallelism a rank only computes the slots routed to its e
 partial outputs are summed across ranks.
 
 Decode-sized batches take the fused path: `moe_route` (RMSNorm + router + top-k + grouped work list, one launch),
-a grouped gate|up GEMV with SwiGLU epilogue and a grouped down GEMV whose last CTA per column tile does the weighted
-combine, the all-reduce across the expert-parallel ranks over peer memory and the residual add
+a grouped gate|up GEMV with SwiGLU epilogue, a grouped down GEMV and the weighted sum into the residual stream.  Under expert
+parallelism with the fused all-reduce the sum is the last CTA's of every column tile of the down GEMV, with the all-reduce over
+peer memory and the residual add
 (the reference runs route, count, scan, scatter, per-expert GEMMs, gather-scale-add and an NCCL all-reduce as
 separate stages: src/v2/compute_stages/stages/MoEExpertComputeStage.cpp, src/v2/models/qwen35moe/Qwen35MoEGraph.cpp:1766-1779).
 Because the residual stream is replicated across the ranks of a tensor-parallel group, "dispatch" needs no transfer:
@@ -66,7 +67,8 @@ def fused_supported(model, L, T: int) -> bool:
 
 
 def moe_forward_fused(model, L, h: torch.Tensor, T: int) -> None:
-    """Three launches per layer: route (+ work list), grouped gate|up + SwiGLU, grouped down + combine + all-reduce + residual."""
+    """Route (+ work list), grouped gate|up + SwiGLU, grouped down, weighted sum into the residual: four launches on the streaming
+    kernels; three where the register path sums in its last CTAs (the fused all-reduce, and calls the streaming kernels do not take)."""
     c, sc = model.cfg, model.scratch
     slab = L.experts
     k = c.n_experts_used

@@ -9,7 +9,9 @@
 //   warp 9     allocates TMEM, issues tcgen05.mma (A = weights, 128 rows; B = activations, BM columns),
 //              releases ring stages with tcgen05.commit.
 // The accumulator is D[n, m] in TMEM (128 lanes x BM fp32 columns): weights sit in the MMA M dimension
-// so a batch-32 decode step wastes nothing, and the same kernel serves prefill with BM = 256.
+// so a batch-32 decode step wastes nothing.  Most calls run on other kernels (launch_gemm_tc: small batches gemm_tc_small.cu, prompts and
+// experts gemm_tc_pair.cu); here remain the fused collectives, forced splits, few rows of narrow and long matrices, Q4_K scales that
+// the short conversion does not take, and more than 256 groups.
 // Skinny problems add split-K over blockIdx.z (fp32 atomics into scratch, last CTA runs the epilogue).
 // Every mbarrier wait is bounded; on a timeout the kernel raises the status word and tears down cleanly.
 //
@@ -658,8 +660,8 @@ cudaError_t launch_gemm_tc(const GemmTcParams& p, cudaStream_t st) {
     if (ks > 1 && (!p.accum || !p.tickets)) ks = 1;
     if (bm <= 128 && !p.rs_on && !p.ag_on && p.groups == 0 && !wide) {
         // Up to 128 rows the product is a stream of weights: the persistent kernel reads it once, every SM the same share.  It
-        // wants the chunks on 16-byte boundaries and work indices of 32 bits; calls of 33 rows or more without these keep
-        // the kernel of large tiles, as they always had it.
+        // wants the chunks on 16-byte boundaries and work indices of 32 bits; calls of 33 rows or more without these, or
+        // with Q4_K scales beyond its conversion, run on the kernel of large tiles.
         const bool fits = !(reinterpret_cast<uintptr_t>(p.w) & 15) && ((unsigned long long)((p.n + 127) / 128) * (p.k / 256) + 1) * 148ull < (1ull << 32);
         if (bm == 32 || (fits && !p.tp)) return launch_gemm_tc_small(p, bm, (p.tickets && p.ksplit != 1) ? 0 : 1, st);
     }

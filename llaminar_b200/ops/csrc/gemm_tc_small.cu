@@ -3,15 +3,15 @@
 //
 // Differences from the large-tile kernel in gemm_tc.cu:
 //   * the packed weight chunks (128 rows x 256 columns, ~14-34 KB) are fetched by one producer warp with 16-byte cp.async
-//     into a deep shared-memory ring (an even number of slots), so HBM latency is hidden by bytes in flight rather than by
+//     into a deep shared-memory ring, so HBM latency is hidden by bytes in flight rather than by
 //     warps waiting on global loads; weights are constants, so under programmatic dependent launch the producer fills the
 //     ring before the wait on the previous kernel;
 //   * 16 dequant warps cooperate on every chunk: warp (g, a) converts the 64-column atom `a` of row group `g`
 //     (lane == row), reading the packed bytes with ld.shared and storing the bf16 values straight into tensor
 //     memory (tcgen05.st), from where the MMA takes its A operand: no shared-memory round trip for the weights.
 //     The converted chunk lives in one of N_SETS operand sets (3; 2 for the formats whose warps alternate);
-//   * two MMA issuer warps each issue half of EVERY chunk (issuer w takes atoms 2w and 2w+1): tcgen05.mma costs ~180
-//     clocks to issue whatever its shape, and issue from different warps overlaps;
+//   * with 32 tokens two MMA issuer warps each issue half of EVERY chunk (issuer w takes atoms 2w and 2w+1): tcgen05.mma costs
+//     ~180 clocks to issue whatever its shape, and issue from different warps overlaps; wider tiles issue from one;
 //   * persistent CTAs (one per SM) walk a contiguous range of (tile, chunk) work ("stream-K"): every SM streams
 //     the same number of bytes, barriers / TMEM are set up once, and two TMEM accumulators let the MMAs of the
 //     next tile start while the previous tile's epilogue drains; the finisher of a split tile loads the parked partial
