@@ -619,7 +619,8 @@ static cudaError_t launch_fmt(const GemmTcParams& p, int bm, int ks, cudaStream_
 // Few rows of a narrow and long matrix leave most pairs without a tile; there the kernel here, which splits K, can be the faster one
 // (its partial sums meet by atomics, in the order they arrive).  Both times in us, as 17 matrices of 512 x 2048 to 5120 x 25600 in four
 // formats showed them at 129 to 512 rows (the rule loses more than 5 % in 7 of 560 calls and 13 % at most):
-//   pairs: 2, and the chunks of the busiest pair at the conversion's rate; the residual's epilogue 4 more
+//   pairs: 2, and the chunks of the busiest pair at the conversion's rate; the residual's epilogue 4 more (as it was when this was fitted;
+//   added in L2 it is not, so residual calls near the line stay on the split a few per cent too long)
 //   split: 22, 1.2 for every chunk of the busiest CTA, 36 for every million outputs (atomics, and the last CTA's epilogue)
 // Examples (pairs, split): 4096 x 12288 Q4_K + residual, 129 rows 71, 53; 256 rows 73, 73; 2560 x 9728 Q8_0, 129 rows 73, 45; 4096 x 4096
 // Q4_K, 129 rows 24, 46.
